@@ -44,6 +44,12 @@ constexpr u32 GMED = 256;       // groups up to this long (and longer than GTINY
 // unsplit, so both rank buffers already hold its head (set only on groups whose input was a small-group list: a group
 // cut out of a larger one by the bucket passes has its parent's head in the other buffer).
 constexpr u32 STABLE = 0x80000000u;
+// Seg.bd bits 24..30 of the groups the rank rounds read: the characters the group's members are known to share when
+// they are more than the round's h (0: h). Round 0's coded keys reach as far as their codewords are short, so groups
+// differ there: on prose a 64-bit key holds 14 characters on average but 8 in the worst group, and doubling from the
+// group's own count instead of the worst one's saves most of a round. (The bucket passes keep their radix digit in
+// the top byte of the groups they split; those start again from h.)
+constexpr u32 DEPTH_SHIFT = 24, DEPTH_MAX = 127;
 
 enum : u8 { C_NONE = 0, C_KS = 1, C_KO = 2, C_LN = 3, C_ONE = 4 };
 
@@ -62,7 +68,8 @@ struct FwdArgs {
     u32 B;
     u32 smax;
     u32 small_group;  // tiles whose groups are all at most this long are sorted by counting, not radix passes
-    u32 lsd_bytes;    // prefix bytes of the LSD round 0 (8, 12 or 16)
+    u32 lsd_bytes;    // key bytes of the LSD round 0 (8, 12 or 16)
+    u32 own_depth;    // groups carry their own depth (round 0 sorted coded keys)
     u32 idn;          // suffix ids of the batch lie in [0, idn)
     u32 rank_passes;  // round 0's ranks: passes of k_seg_rank over id ranges, or 0: written by the emit kernels
     u32 warp_path;    // 1: tiles without a group longer than WARP_GROUP belong to the warp-level kernel
@@ -72,6 +79,7 @@ struct FwdArgs {
     unsigned long long *lit[2];  // round 0: (key group << 32 | id) items, aliasing lval[q] and lhi[q]
     u64 *lstat;
     u32 *lhist, *ltile, *segagg;
+    u32 *ctab;   // round 0: every block's code table
     u32 *lbase;  // round 0: per block and digit slot, the pass's first position of every digit
     u32 spin_limit;
     // repeat chains (rank rounds >= chain_from): bit x of cbits = the group of suffix x continues at x + 1;
@@ -93,6 +101,16 @@ __device__ __forceinline__ u64 blk_end(const FwdArgs &a, u32 b) {
     return (u64)B.off + B.n;
 }
 __device__ __forceinline__ u32 seg_depth(u32 bd) { return bd >> 24; }
+// The characters members of group bd share in a round that has sorted h, and the bits of the groups it splits into
+// (they share h more, by the ranks that sorted them; 0 where the next round's 2h is as much).
+__device__ __forceinline__ u32 seg_h(u32 bd, u32 h) {
+    const u32 d = (bd >> DEPTH_SHIFT) & DEPTH_MAX;
+    return max(d, h);
+}
+__device__ __forceinline__ u32 next_depth(u32 bd, u32 h) {
+    const u32 d = (bd >> DEPTH_SHIFT) & DEPTH_MAX, nd = min(d + h, DEPTH_MAX);
+    return d > h && nd > 2 * h ? nd << DEPTH_SHIFT : 0u;
+}
 
 // Depth of the first bucket pass of a rank-round group from the OR/AND of its keys: the byte of the highest
 // varying bit (3 when all keys are equal, which then finishes the group in one pass).
@@ -130,13 +148,12 @@ __device__ __forceinline__ void resolve_byte(const FwdArgs &a, u32 *isa_nxt, u32
     if (a.SA) a.SA[(u64)B.off + p] = id - B.off;
     if (ridx < a.cap_res) { res.eid[ridx] = id; res.ekey[ridx] = p; }
 }
-// As resolve, for round 0: no resolved-list entry (round 1's fixup copies the whole rank buffer) and the rank only
-// when the caller writes it.
+// As resolve, for round 0: no resolved-list entry (round 1's fixup copies the whole rank buffer), the rank only when
+// the caller writes it, and no L column (k_seg_count wrote it).
 __device__ __forceinline__ void resolve_round0(const FwdArgs &a, u32 *isa_nxt, u32 id, u32 p, u32 b) {
     BlockInfo B = a.blk[b];
     if (!KGB_OK(id < a.cap_n && p < B.n && id >= B.off && id - B.off < B.n, &a.ctl->err, E_RANK)) return;
     if (isa_nxt) isa_nxt[id] = p;
-    a.L[(u64)B.off + b + p + 1] = id == B.off ? 0 : __ldg(a.T + id - 1);
     if (a.SA) a.SA[(u64)B.off + p] = id - B.off;
 }
 __device__ __forceinline__ void resolve(const FwdArgs &a, u32 *isa_nxt, u32 id, u32 p, u32 b, ListView res,
@@ -269,7 +286,7 @@ __global__ void __launch_bounds__(TPB, TileTraits<PREFIX, TILE>::MINB) k_tile_so
                     key = in.ekey[E0 + x];
                 } else {
                     const BlockInfo B = a.blk[seg_blk(S.lblk[lo])];
-                    key = rank_key(isa_cur, id, h, (u64)B.off + B.n);
+                    key = rank_key(isa_cur, id, seg_h(S.lblk[lo], h), (u64)B.off + B.n);
                 }
                 k[j] = key;
                 hi[j] = lo;
@@ -503,7 +520,7 @@ __global__ void __launch_bounds__(TPB, TileTraits<PREFIX, TILE>::MINB) k_tile_so
                 KGB_GUARD(id < a.cap_n, &a.ctl->err, E_RANK) isa_nxt[id] = head;
             }
             const u32 len = (u32)S.klo[gfirst];
-            const u32 sbd = seg_blk(bd) | (!PREFIX && !KEYED && unsplit ? STABLE : 0u);
+            const u32 sbd = seg_blk(bd) | (!PREFIX && !KEYED ? next_depth(bd, h) | (unsplit ? STABLE : 0u) : 0u);
             if (len <= GTINY) {
                 KGB_GUARD(pebase + ep < a.cap_n, &a.ctl->err, E_LIST) outp.eid[pebase + ep] = id;
                 if (st[j]) gp++;
@@ -664,7 +681,7 @@ __global__ void __launch_bounds__(TPB, 3) k_tile_warp(FwdArgs a) {
                             if (rem < 8) kk &= ~0ull << (8 * (8 - rem));
                             keys[q] = (KeyT)kk;
                         } else {
-                            keys[q] = (KeyT)rank_key(isa_cur, ids[q], h, end);
+                            keys[q] = (KeyT)rank_key(isa_cur, ids[q], seg_h(S.lbd[sgs[q]], h), end);
                         }
                     }
                 }
@@ -787,7 +804,7 @@ __global__ void __launch_bounds__(TPB, 3) k_tile_warp(FwdArgs a) {
                     if (!((bd & STABLE) && unsplit)) {
                         KGB_GUARD(id < a.cap_n, &a.ctl->err, E_RANK) isa_nxt[id] = head;
                     }
-                    const u32 sbd = seg_blk(bd) | (!PREFIX && !KEYED && unsplit ? STABLE : 0u);
+                    const u32 sbd = seg_blk(bd) | (!PREFIX && !KEYED ? next_depth(bd, h) | (unsplit ? STABLE : 0u) : 0u);
                     if (tiny) {
                         KGB_GUARD(pebase + my_ep < a.cap_n, &a.ctl->err, E_LIST) outp.eid[pebase + my_ep] = id;
                         if (en) {
@@ -1029,11 +1046,12 @@ __global__ void __launch_bounds__(TPB, 4) k_group_thread(FwdArgs a) {
         // at least as far, so it takes that key instead (one gather per member either way). Shorter chains, and
         // rounds without chains, take the doubling key.
         u32 d = 0;
+        const u32 gh = seg_h(g.bd, h);
         if (len >= 2 && chain_on(a)) d = chain_end(a, v[0]) - v[0];
-        const bool by_chain = d >= h;
+        const bool by_chain = d >= gh;
 #pragma unroll
         for (u32 q = 0; q < GTINY; q++)
-            k[q] = q >= len ? 0xFFFFFFFFu : by_chain ? chain_key(isa_cur, v[q], d, end) : rank_key(isa_cur, v[q], h, end);
+            k[q] = q >= len ? 0xFFFFFFFFu : by_chain ? chain_key(isa_cur, v[q], d, end) : rank_key(isa_cur, v[q], gh, end);
         {
             const u32 lq = gq.len <= GTINY && (u64)gq.start + gq.len <= nslots && s + stride < nseg ? gq.len : 0u;
 #pragma unroll
@@ -1111,7 +1129,7 @@ __global__ void __launch_bounds__(TPB, 4) k_group_thread(FwdArgs a) {
             if (en) {
                 Seg ng_;
                 ng_.len = q - rs + 1; ng_.start = g.start + rs; ng_.head = head;
-                ng_.bd = b | (unsplit ? STABLE : 0u);
+                ng_.bd = b | next_depth(g.bd, h) | (unsplit ? STABLE : 0u);
                 KGB_GUARD(gi < a.cap_segt, &a.ctl->err, E_SEG) out.seg[gi] = ng_;
                 gi++;
             }
@@ -1128,17 +1146,39 @@ __global__ void __launch_bounds__(TPB, 4) k_group_thread(FwdArgs a) {
 // lengths and offsets in the next lists, once to emit ranks, finished suffixes and runs (tiny ones to the tiny list,
 // the others to the medium list).
 
-// Raw keys of the medium list: mkey[x] = ISA[eid[x] + h] (clamped into the rank buffer; corrected per block later).
+// Raw keys of the medium list: mkey[x] = ISA[eid[x] + h] (clamped into the rank buffer; corrected per block later), h
+// the characters the element's group shares. After a raw round 0 that is the same for all, and the list is gathered
+// flat, every load independent; after a coded one each warp takes whole groups, the next group's descriptor loaded
+// ahead (0.15 ms flat against 0.19 by groups for the 9.5 M elements of round 1 on 64 MiB of prose).
 __global__ void __launch_bounds__(TPB) k_mkeys(FwdArgs a) {
     const Ctl *ctl = a.ctl;
     const u32 rpar = ctl->rpar, h = ctl->h;
     const ListView in = a.lists[L_M0 + rpar];
     const u32 nelem = min((u32)ctl->cnt[L_M0 + rpar], (u32)a.cap_n);
+    const u32 nseg = min((u32)(ctl->cnt[L_M0 + rpar] >> 32), (u32)a.cap_segm);
     const u32 *isa_cur = a.isa[rpar];
     u32 *mk = a.lval[0];
-    for (u32 x = blockIdx.x * TPB + threadIdx.x; x < nelem; x += gridDim.x * TPB) {
-        const u64 j = (u64)in.eid[x] + h;
-        mk[x] = j < a.cap_n ? __ldg(isa_cur + j) : 0u;
+    if (!a.own_depth) {
+        for (u32 x = blockIdx.x * TPB + threadIdx.x; x < nelem; x += gridDim.x * TPB) {
+            const u64 j = (u64)in.eid[x] + h;
+            mk[x] = j < a.cap_n ? __ldg(isa_cur + j) : 0u;
+        }
+        return;
+    }
+    const u32 lane = lane_id();
+    const u32 gw = blockIdx.x * (TPB / 32) + warp_id(), nw = gridDim.x * (TPB / 32);
+    Seg gq = {0, 0, 0, 0};
+    if (gw < nseg) gq = in.seg[gw];
+    for (u32 s = gw; s < nseg; s += nw) {
+        const Seg g = gq;
+        if (s + nw < nseg) gq = in.seg[s + nw];
+        const u32 len = g.len <= GMED && (u64)g.start + g.len <= nelem ? g.len : 0u;
+        const u32 gh = seg_h(g.bd, h);
+#pragma unroll 4
+        for (u32 x = lane; x < len; x += 32) {
+            const u64 j = (u64)in.eid[g.start + x] + gh;
+            mk[g.start + x] = j < a.cap_n ? __ldg(isa_cur + j) : 0u;
+        }
     }
 }
 
@@ -1175,7 +1215,7 @@ __global__ void __launch_bounds__(TPB) k_group_warp(FwdArgs a) {
             if (lane == 0) atomicOr(&a.ctl->err, E_SEG);
             continue;
         }
-        const u32 b = seg_blk(g.bd);
+        const u32 b = seg_blk(g.bd), gh = seg_h(g.bd, h);
         const u64 end = blk_end(a, b);
         if (len <= 32) {
             // ---- counting sort, one member per lane (position = keys below + equal keys before)
@@ -1183,7 +1223,7 @@ __global__ void __launch_bounds__(TPB) k_group_warp(FwdArgs a) {
             if (lane < len) {
                 id = in.eid[g.start + lane];
                 const u32 d = (u32)(end - id);
-                kx = h < d ? mk[g.start + lane] + h : d - 1;
+                kx = gh < d ? mk[g.start + lane] + gh : d - 1;
             }
             u32 below = 0;
             for (u32 y = 0; y < len; y++) {
@@ -1199,7 +1239,7 @@ __global__ void __launch_bounds__(TPB) k_group_warp(FwdArgs a) {
                 if (q < len) {
                     id = in.eid[g.start + q];
                     const u32 d = (u32)(end - id);
-                    kx = h < d ? mk[g.start + q] + h : d - 1;
+                    kx = gh < d ? mk[g.start + q] + gh : d - 1;
                 }
                 K[q] = kx;
                 V[q] = id;
@@ -1263,7 +1303,7 @@ __global__ void __launch_bounds__(TPB) k_group_warp(FwdArgs a) {
         __syncwarp();
         // ---- emit
         const bool skip_rank = (g.bd & STABLE) && unsplit;
-        const u32 sbd = b | (unsplit ? STABLE : 0u);
+        const u32 sbd = b | next_depth(g.bd, h) | (unsplit ? STABLE : 0u);
         carry = 0;
         u32 r1 = 0;
         for (u32 c0 = 0; c0 < len; c0 += 32) {
@@ -1376,7 +1416,7 @@ __global__ void __launch_bounds__(TPB) k_keygen(FwdArgs a) {
                 const bool sel = x >= bound;
                 const BlockInfo &B = sel ? B1 : B0;
                 const u32 id = in.eid[x];
-                const u32 key = rank_key(isa, id, h, (u64)B.off + B.n);
+                const u32 key = rank_key(isa, id, seg_h((sel ? g1 : g0).bd, h), (u64)B.off + B.n);
                 in.ekey[x] = key;
                 if (sel) { or1 |= key; and1 &= key; } else { or0 |= key; and0 &= key; }
             }
@@ -1841,6 +1881,7 @@ void FwdEngine::layout(u64 ncap, u32 bcap, u32 icap, bool want_sa, Add add) {
     add((void **)&d_segbits, n / 8 + 64);
     add((void **)&d_lhist, (size_t)bcap * 256 * 4);  // byte histogram of every block
     add((void **)&d_lbase, (size_t)bcap * NSLOT * 256 * 4);
+    add((void **)&d_ctab, (size_t)bcap * CODE_ROW * 4);  // code table of every block
     add((void **)&d_ltile, NSLOT * 4);
     add((void **)&d_segagg, stiles * 8 * 4);
     // repeat chains: a bit per id, its next-zero table per word and per tile of words
@@ -1935,6 +1976,7 @@ void FwdEngine::set_caps(FwdArgs &a) const {
     for (int q = 0; q < 2; q++) a.lit[q] = reinterpret_cast<unsigned long long *>(d_lval[q]);
     a.segbits = d_segbits;
     a.lstat = d_lstat; a.lhist = d_lhist; a.ltile = d_ltile; a.segagg = d_segagg; a.lbase = d_lbase;
+    a.ctab = d_ctab;
     a.cbits = d_cbits; a.cnz = d_cnz; a.ctn = d_ctn;
     a.cwords = (u32)(N / 32 + 2);
     a.ctiles = (a.cwords + NZ_TILE - 1) / NZ_TILE;
@@ -1942,6 +1984,7 @@ void FwdEngine::set_caps(FwdArgs &a) const {
     a.spin_limit = 1u << 22;
     a.small_group = (u32)cfg.small_group;
     a.lsd_bytes = (u32)cfg.lsd_bytes;
+    a.own_depth = lsd_enabled() && lsd_coded(a);
     a.idn = (u32)N;
     {
         // the emit kernels' rank writes stay within one block's ids at a time (the sorted order is block-major), so
@@ -2058,7 +2101,7 @@ int FwdEngine::setup_round0(cudaStream_t s) {
     c.cnt[L_L0] = ((u64)seg_l.size() << 32) | el;
     c.maxrounds = (u32)ceil_log2(maxn) + 3;
     c.seq = ++call_seq;
-    c.h0 = lsd_enabled() ? (u32)cfg.lsd_bytes : 8u;
+    c.h0 = 8;  // the tile path's prefix; the LSD round 0 sets its own
     c.lsd_tiles = lt_b;
     c.idn = (u32)N;  // N is the batch's extent: max over blocks of off + n
     KGB_CHECK(cudaMemcpyAsync(d_blk, bi.data(), B * sizeof(BlockInfo), cudaMemcpyHostToDevice, s));
@@ -2111,7 +2154,7 @@ static int warp_smem() { return (int)sizeof(WarpSmem<TILE, typename TileTraits<P
 
 struct Launcher {
     cudaStream_t s;
-    int grid_tile, grid_msd, grid_scan, tile_cap, grid_tile_prefix, grid_warp, grid_lsd;
+    int grid_tile, grid_msd, grid_scan, tile_cap, grid_tile_prefix, grid_warp, grid_lsd, grid_keys;
     long long *launches;
     Profiler *prof;
     template <typename K, typename... Args>
@@ -2152,7 +2195,8 @@ static int set_tile_attrs(int tile) {
         KGB_CHECK(cudaFuncSetAttribute(k_tile_warp<false, false, 8192>, cudaFuncAttributeMaxDynamicSharedMemorySize, warp_smem<false, 8192>()));
         KGB_CHECK(cudaFuncSetAttribute(k_tile_warp<false, true, 8192>, cudaFuncAttributeMaxDynamicSharedMemorySize, warp_smem<false, 8192>()));
     }
-    KGB_CHECK(cudaFuncSetAttribute(k_lsd_pass, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lsd_smem()));
+    KGB_CHECK(cudaFuncSetAttribute(k_lsd_pass<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lsd_smem()));
+    KGB_CHECK(cudaFuncSetAttribute(k_lsd_pass<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lsd_smem()));
     g_attr_done[idx] = true;
     return 0;
 }
@@ -2242,8 +2286,17 @@ static cudaError_t enq_lsd_keys(Launcher &L, const FwdArgs &a) {
     if ((e = L.go(k_lsd_begin, L.grid_msd, 256, 0, a))) return e;
     L.tag(K_LSD_KEY0, 0);
     if ((e = L.go(k_lsd_key0, L.grid_msd, TPB, 0, a))) return e;
+    const int gb = std::min<int>((int)a.B, L.grid_msd);
+    if (!lsd_coded(a)) {
+        L.tag(K_LSD_HIST, 0);
+        return L.go(k_lsd_hist0, gb, TPB, 0, a);
+    }
+    L.tag(K_LSD_CODE, 0);
+    if ((e = L.go(k_lsd_code, gb, TPB, 0, a))) return e;
+    L.tag(K_LSD_KEYS, 0);
+    if ((e = L.go(k_lsd_keys, std::min(L.grid_lsd, L.grid_keys), TPB, 0, a))) return e;
     L.tag(K_LSD_HIST, 0);
-    return L.go(k_lsd_hist0, std::min<int>((int)a.B, L.grid_msd), TPB, 0, a);
+    return L.go(k_lsd_base, gb, TPB, 0, a);
 }
 static cudaError_t enq_lsd_sort_seg(Launcher &L, const FwdArgs &a, u32 slots, u32 m_tag) {
     cudaError_t e;
@@ -2254,12 +2307,14 @@ static cudaError_t enq_lsd_sort_seg(Launcher &L, const FwdArgs &a, u32 slots, u3
         if (!((slots >> slot) & 1)) continue;
         L.tag(K_LSD_PASS, m_tag);
         if (L.prof) L.prof->pass = slot;
-        if ((e = L.go(k_lsd_pass, L.grid_lsd, TPB, lsd_smem(), a, slot)))
+        if ((e = lsd_coded(a) ? L.go(k_lsd_pass<true>, L.grid_lsd, TPB, lsd_smem(), a, slot)
+                              : L.go(k_lsd_pass<false>, L.grid_lsd, TPB, lsd_smem(), a, slot)))
             return e;
     }
     if (L.prof) L.prof->pass = -1;
     L.tag(K_SEG_COUNT, m_tag);
-    if ((e = L.go(k_seg_count, L.grid_msd, TPB, 0, a))) return e;
+    if ((e = lsd_coded(a) ? L.go(k_seg_count<true>, L.grid_msd, TPB, 0, a) : L.go(k_seg_count<false>, L.grid_msd, TPB, 0, a)))
+        return e;
     L.tag(K_SEG_SCAN, m_tag);
     if ((e = L.go(k_seg_scan, 1, 1024, 0, a))) return e;
     L.tag(K_SEG_EMIT1, m_tag);
@@ -2296,7 +2351,7 @@ int FwdEngine::run_plain(cudaStream_t s) {
                           B, smax);
     set_caps(a);
     prof.reset();
-    Launcher L{s, grid_tile, grid_msd, grid_scan, cfg.tile_cap, grid_tile_prefix, grid_warp, grid_lsd, &stats.launches, prof.on ? &prof : nullptr};
+    Launcher L{s, grid_tile, grid_msd, grid_scan, cfg.tile_cap, grid_tile_prefix, grid_warp, grid_lsd, grid_keys, &stats.launches, prof.on ? &prof : nullptr};
     auto cnt_e = [&](u32 l) { return (u32)h_ctl->cnt[l]; };
     auto cnt_s = [&](u32 l) { return (u32)(h_ctl->cnt[l] >> 32); };
     auto read_ctl = [&]() -> int {
@@ -2486,7 +2541,7 @@ int FwdEngine::build_graph(cudaStream_t s) {
     FwdArgs ar = a;
     ar.hcond = (unsigned long long)hround;
     long long dummy = 0;
-    Launcher L{s, grid_tile, grid_msd, grid_scan, cfg.tile_cap, grid_tile_prefix, grid_warp, grid_lsd, &dummy, nullptr};
+    Launcher L{s, grid_tile, grid_msd, grid_scan, cfg.tile_cap, grid_tile_prefix, grid_warp, grid_lsd, grid_keys, &dummy, nullptr};
     Deps deps;
     if (lsd) {
         if (int rc = capture_into(s, graph, deps, [&]() -> cudaError_t {
@@ -2531,6 +2586,7 @@ int FwdEngine::run(cudaStream_t s, bool use_graph) {
     grid_tile_prefix = sm_count * (cfg.tile_cap == 4096 ? 2 : 1);
     grid_warp = sm_count * (cfg.tile_cap == 4096 ? 4 : 2);
     grid_lsd = (int)((N + LSD_TILE - 1) / LSD_TILE + B);  // at least the batch's sort tiles (one partial per block)
+    grid_keys = sm_count * 4;  // what the shared memory of k_lsd_keys admits
     grid_msd = sm_count * cfg.msd_ctas;
     grid_scan = sm_count * 4;
     // the host-side round-0 layout borrows the cursor/dest rows; they are rewritten by every bucket scan

@@ -18,7 +18,8 @@ struct BlockInfo {
 
 // A segment of an element list: `len` consecutive elements starting at `start` that form one group (equal sort
 // keys so far) whose first member sits at suffix-array position `head` of block `bd & 0xFFFFFF`. The top byte of
-// `bd` holds the next radix digit for segments still being split by the bucket passes.
+// `bd` holds the next radix digit for segments still being split by the bucket passes, else the group's shared
+// characters and the STABLE flag (see fwd.cu).
 struct Seg {
     u32 start, len, head, bd;
 };
@@ -57,7 +58,7 @@ struct Ctl {
     u64 tile_elems[2];  // elements sorted so far by the block-level and the warp-level tile kernels (statistics)
     // round 0 as an LSD radix sort
     u32 lsd_act;        // bit s: digit slot s varies (a pass runs for it)
-    u32 h0;             // characters round 0 sorts (the first rank round's h)
+    u32 h0;             // characters round 0 has sorted in every group it leaves (the first rank round's h)
     u32 m;              // suffixes sorted
     u32 seq;            // call sequence number (tags the look-back words of the radix passes)
     u32 p_alloc;        // slots taken so far in the tiny-group id array (shared by both parities, never reused)
@@ -73,7 +74,7 @@ struct FwdConfig {
     int small_group = 64; // tiles whose groups are all at most this long skip the radix passes (counting sort)
     int warp_path = 1;    // tiles whose groups are all <= 32 long go to the warp-level kernel
     int lsd_round0 = 1;   // round 0 as one LSD radix sort of all suffixes; 0: bucket passes + tiles over 8-byte prefixes
-    int lsd_bytes = 16;   // prefix bytes the LSD round 0 sorts (8, 12 or 16)
+    int lsd_bytes = 16;   // bytes of the coded prefix the LSD round 0 sorts (8, 12 or 16)
     int chain_from = 1;   // first rank round whose tiny groups may be ordered along their repeat chains (0: never)
 };
 // Fields of FwdConfig a caller set explicitly (they override the tuning table).
@@ -169,6 +170,7 @@ class FwdEngine {
     u32 *d_lval[2] = {nullptr, nullptr}, *d_lhi[2] = {nullptr, nullptr};
     u64 *d_lstat = nullptr;
     u32 *d_lbase = nullptr;
+    u32 *d_ctab = nullptr;
     u32 *d_lhist = nullptr, *d_ltile = nullptr, *d_segagg = nullptr, *d_segbits = nullptr;
     u32 *d_cbits = nullptr, *d_cnz = nullptr, *d_ctn = nullptr;  // repeat chains
     u64 lsd_tiles_cap = 0, seg_tiles_cap = 0;
@@ -204,7 +206,7 @@ class FwdEngine {
     GraphKey seen_key{};
     bool seen_valid = false;
     int sm_count = 0;
-    int grid_tile = 0, grid_msd = 0, grid_scan = 0, grid_tile_prefix = 0, grid_warp = 0, grid_lsd = 0;
+    int grid_tile = 0, grid_msd = 0, grid_scan = 0, grid_tile_prefix = 0, grid_warp = 0, grid_lsd = 0, grid_keys = 0;
 };
 
 }  // namespace kgb

@@ -1,21 +1,29 @@
-// Round 0 of the forward sort as one LSD radix sort: the suffixes of each block of the batch are sorted by their
-// zero-padded W-byte prefix, W = 16 (or 12 or 8), with one pass per varying key byte (single-pass scatter with decoupled
-// look-back), then a segmentation turns the sorted order into ranks, finished suffixes and the rank rounds' groups
-// (tiny, medium, small and large lists). The sort tiles never straddle two blocks: every block's suffixes keep their
-// own range of the dense order (the block's soff onward), a pass takes each tile's digit bases from its own block's
-// counts and looks back only over the block's earlier tiles, so the block index is neither carried nor sorted. The
-// passes move 8-byte (id, key) items whose key is the 4-byte group of prefix bytes the passes of that group sort:
-// the first pass builds its items from the text (ids still in text order, so the loads coalesce), and the last pass
-// of a group writes the next group's key, gathered from the text (which stays in L2 at these sizes), so each pass
-// reads and writes 16 B per suffix. The segmentation compares the whole W-byte prefixes, read from the text. Sorting
-// 16 bytes here replaces the first rank round (which would take the groups from 8 to 16 bytes) with eight passes over
-// all suffixes. Included by fwd.cu inside namespace kgb, after the kernels it shares (FwdArgs, resolve, tile-map
-// writers).
+// Round 0 of the forward sort as one LSD radix sort: the suffixes of each block of the batch are sorted by a W-byte
+// key, with one pass per varying key byte (single-pass scatter with decoupled look-back), then a segmentation turns the
+// sorted order into ranks, finished suffixes and the rank rounds' groups (tiny, medium, small and large lists). The
+// sort tiles never straddle two blocks: every block's suffixes keep their own range of the dense order (the block's
+// soff onward), a pass takes each tile's digit bases from its own block's counts and looks back only over the block's
+// earlier tiles, so the block index is neither carried nor sorted. The passes move 8-byte (id, key) items whose key is
+// the 4-byte group of key bytes the passes of that group sort; the last pass of a group writes the next group's key
+// instead of its own, so each pass reads and writes 16 B per suffix. Included by fwd.cu inside namespace kgb, after the
+// kernels it shares (FwdArgs, resolve, tile-map writers).
+//
+// Raw keys (W = 16 or 12): the first W bytes of the suffix, zero-padded. The first pass builds its items from the text
+// (ids still in text order, so the loads coalesce), a group's last pass gathers the next group's bytes from the text.
+//
+// Coded keys (W = 8): the first 64 bits of the suffix written in an order-preserving prefix code of its block's bytes.
+// A block's bytes take codewords of 1..CODE_MAX bits from a weight-balanced binary tree over its byte histogram
+// (alphabetic, so comparing encoded suffixes as bit strings compares the suffixes; the smallest byte's codeword is all
+// zeros and zeros follow the block's end, so a suffix that ends sorts with the ones that go on in smallest bytes, in
+// one group). Suffixes with equal keys share as many bytes as their key holds whole codewords; the smallest such count
+// over the groups of two or more is what round 0 has sorted (Ctl::h0), and each group carries its own. Raw bytes take
+// 8 bits each whatever they hold, coded ones about their order-0 entropy (prose 4.7 bits, log lines 5.1, ACGT 2.0,
+// 64-symbol Markov 6.0), so eight passes reach 10-32 characters where sixteen reach 16.
 #pragma once
 // (included inside namespace kgb)
 
 constexpr int LSD_IPT = 16, LSD_TILE = TPB * LSD_IPT;  // elements per sort tile
-// digit slots: slot s sorts prefix byte 15 - s, carried in key group (15 - s) / 4 (bytes 4g..4g+3, big-endian)
+// digit slots: slot s sorts key byte 15 - s, carried in key group (15 - s) / 4 (bytes 4g..4g+3, big-endian)
 constexpr int NSLOT = 16;
 static_assert(NSLOT <= 32, "the look-back epoch holds the slot in 5 bits");
 constexpr int SEG_IPT = 16, SEG_TILE = TPB * SEG_IPT;  // positions per segmentation tile (SEG_IPT <= 32)
@@ -25,42 +33,109 @@ constexpr u64 ST_AGG = 1ull << 30, ST_PRE = 2ull << 30, ST_VAL = (1ull << 30) - 
 constexpr u64 ST_EPOCH = 0xFFFFFFFF00000000ull;
 constexpr int LB_WIN = 8;  // look-back window (predecessor words read per step)
 
+// Which keys: the tuning table's choice per batch size, by measurement. Coded keys halve the passes but compare more in
+// the segmentation and leave slightly larger groups. Coded against the best raw width, all kernels of the call: 1 MiB
+// Markov block 0.31 ms against 0.44, 64 slices of 512 KiB prose 4.8 against 5.3, 64 mixed blocks (216 MB) 31.7 against
+// 33.9; on single blocks of prose over 32 MiB the deeper raw 16 bytes win (64 MiB: 15.5 against 16.1), because there
+// the rank rounds' gathers miss L2 and every active suffix they are left costs fifteen passes' worth.
+__host__ __device__ __forceinline__ bool lsd_coded(const FwdArgs &a) { return a.lsd_bytes == 8; }
 __device__ __forceinline__ u32 active_slots(const Ctl *c) { return c->lsd_act; }  // bit s: slot s varies
 
+// A block's code table: entry c holds byte c's codeword left-aligned in bits 31..20 and its length in bits 4..0, entry
+// CODE_PAD the symbol past the block's end (zeros of the smallest byte's length), entry CODE_MIN the smallest byte.
+constexpr u32 CODE_MAX = 12, CODE_BITS = 0xFFF00000u, CODE_PAD = 256, CODE_MIN = 257, CODE_ROW = 260;  // words
+
+// The 16 text bytes from position q < end on, and the byte before them. Random text reads are bound by the lines a
+// warp's loads touch (one a cycle and SM), not by their bytes, so they take two aligned 16-byte granules instead of
+// three 8-byte words. Every granule read holds a byte of the block: it ends at most 15 bytes past the block and begins
+// in the granule of its first byte.
+struct Text16 {
+    u64 w, w2;        // bytes q..q+7 and q+8..q+15
+    u8 before;        // byte q - 1 when it lies in the first granule
+    bool has_before;  // (q not at a granule's start)
+};
+__device__ __forceinline__ Text16 text16(const u8 *__restrict__ T, u64 q, u64 end) {
+    const u8 *p = T + q;
+    const u32 s = (u32)(reinterpret_cast<uintptr_t>(p) & 15u);
+    const ulonglong2 *g = reinterpret_cast<const ulonglong2 *>(p - s);
+    Text16 r;
+    const ulonglong2 x = __ldg(g);
+    ulonglong2 y = make_ulonglong2(0, 0);
+    if (q + (16 - s) < end) y = __ldg(g + 1);
+    const u32 h = (s & 7) * 8;
+    const u64 a = s & 8 ? x.y : x.x, b = s & 8 ? y.x : x.y, c = s & 8 ? y.y : y.x;
+    r.w = h ? (a >> h) | (b << (64 - h)) : a;
+    r.w2 = h ? (b >> h) | (c << (64 - h)) : b;
+    r.has_before = s != 0;
+    r.before = (u8)((((s - 1) & 8) ? x.y : x.x) >> (8 * ((s - 1) & 7)));
+    return r;
+}
+// As text16, with every byte past the block's end replaced by the block's smallest byte (what zeros past the end of a
+// coded suffix read as).
+__device__ __forceinline__ Text16 text16_padded(const u8 *__restrict__ T, u64 q, u64 end, u32 smallest) {
+    const u64 fill = 0x0101010101010101ull * smallest;
+    Text16 r;
+    r.w = r.w2 = fill;
+    r.before = 0;
+    r.has_before = false;
+    if (q >= end) return r;
+    r = text16(T, q, end);
+    const u64 rem = end - q;
+    if (rem < 8) r.w = (r.w & ~(~0ull << (8 * rem))) | fill << (8 * rem);
+    if (rem <= 8) r.w2 = fill;
+    else if (rem < 16) r.w2 = (r.w2 & ~(~0ull << (8 * (rem - 8)))) | fill << (8 * (rem - 8));
+    return r;
+}
+
+// The first 32 NG key bits of the suffix at q into k[], and into m[] the bits where a codeword ends. Eight symbols a
+// step: their look-ups are independent, and codewords are joined in pairs before they enter the bit windows. The loop
+// ends: every table entry is at least one bit long.
+template <int NG>
+__device__ __forceinline__ void lsd_encode(const u8 *__restrict__ T, const u32 *tab, u64 q, u64 end, u32 *k, u32 *m) {
+    u32 hi = 0, lo = 0, mhi = 0, mlo = 0, fill = 0;
+    for (int g = 0; g < NG; q += 8) {
+        u64 w = 0;
+        if (q < end) w = text16(T, q, end).w;
+        u32 e[8];
+#pragma unroll
+        for (int j = 0; j < 8; j++) e[j] = tab[q + j < end ? (u32)(w >> (8 * j)) & 0xFFu : CODE_PAD];
+#pragma unroll
+        for (int j = 0; j < 8; j += 2) {
+            // (the funnel shift takes its count modulo 32: a length in the low five bits; two lengths sum below 32)
+            const u32 pair = (e[j] & CODE_BITS) | __funnelshift_r(e[j + 1] & CODE_BITS, 0u, e[j]);
+            const u32 l = (e[j] + e[j + 1]) & 31u, ends = 1u << (32 - (e[j] & 31u)) | 1u << (32 - l);
+            hi |= pair >> fill;
+            lo |= __funnelshift_r(0u, pair, fill);
+            mhi |= ends >> fill;
+            mlo |= __funnelshift_r(0u, ends, fill);
+            fill += l;
+            if (fill >= 32) {
+#pragma unroll
+                for (int x = 0; x < NG; x++) if (x == g) { k[x] = hi; m[x] = mhi; }
+                g++;
+                hi = lo; mhi = mlo;
+                lo = mlo = 0;
+                fill -= 32;
+            }
+        }
+    }
+}
 // The zero-padded 8-byte text word at position q of a block ending at end, as a big-endian word (0 past the end).
-__device__ __forceinline__ u64 lsd_key(const u8 *__restrict__ T, u64 q, u64 end) {
+__device__ __forceinline__ u64 lsd_word(const u8 *__restrict__ T, u64 q, u64 end) {
     if (q >= end) return 0;
     u64 k = load_be64(T, q);
     const u64 rem = end - q;
     if (rem < 8) k &= ~0ull << (8 * (8 - rem));
     return k;
 }
-// The zero-padded 16-byte prefix at position q as two big-endian words (k: bytes 0-7, k2: bytes 8-15, 0 past the
-// block end), from three aligned 8-byte loads; `two` false: k2 = 0 and only two loads. The third load is made only
-// when byte q + 8 lies in the block, so no load reaches more than 15 bytes past the block's end (the padding that
-// callers of the engine guarantee).
-__device__ __forceinline__ void lsd_key16(const u8 *__restrict__ T, u64 q, u64 end, bool two, u64 &k, u64 &k2) {
-    k = k2 = 0;
-    if (q >= end) return;
-    const u64 *p = reinterpret_cast<const u64 *>(T + (q & ~7ull));
-    const u64 a = __ldg(p), b = __ldg(p + 1), c = two && end - q > 8 ? __ldg(p + 2) : 0ull;
-    const u32 s = (u32)(q & 7) * 8;
-    const u64 w0 = s ? (a >> s) | (b << (64 - s)) : a, w1 = s ? (b >> s) | (c << (64 - s)) : b;
-    auto be = [](u64 w) {
-        return ((u64)__byte_perm((u32)w, 0, 0x0123) << 32) | (u64)__byte_perm((u32)(w >> 32), 0, 0x0123);
-    };
-    const u64 rem = end - q;
-    k = be(w0);
-    if (rem < 8) k &= ~0ull << (8 * (8 - rem));
-    if (two && rem > 8) {
-        k2 = be(w1);
-        if (rem < 16) k2 &= ~0ull << (8 * (16 - rem));
-    }
+// Raw keys: key group g (prefix bytes 4g..4g+3) of the suffix at id, big-endian, zero past the block end.
+__device__ __forceinline__ u32 lsd_raw_group(const u8 *__restrict__ T, u32 id, u32 g, u64 end) {
+    return (u32)(lsd_word(T, (u64)id + 4 * g, end) >> 32);
 }
-// Key group g (prefix bytes 4g..4g+3) of the suffix at id, big-endian, zero past the block end.
-__device__ __forceinline__ u32 lsd_group(const u8 *__restrict__ T, u32 id, u32 g, u64 end) {
-    return (u32)(lsd_key(T, (u64)id + 4 * g, end) >> 32);
-}
+// Coded keys: key group g (0 or 1) of every suffix, and the whole codewords of its key, in text order (dense order of
+// the batch). They live in lists that are empty in round 0, the last group's in the buffer the first pass reads from.
+__device__ __forceinline__ u32 *lsd_keys_of(const FwdArgs &a, u32 g) { return g ? a.lval[0] : a.lists[L_KS].eid; }
+__device__ __forceinline__ u8 *lsd_whole_of(const FwdArgs &a) { return reinterpret_cast<u8 *>(a.lists[L_M0].eid); }
 // Key group of slot s.
 __device__ __forceinline__ u32 lsd_slot_group(int slot) { return (15u - (u32)slot) >> 2; }
 
@@ -95,11 +170,15 @@ __device__ __forceinline__ LsdTile lsd_tile(const FwdArgs &a, u32 t) {
     return r;
 }
 
-// Start: clear the blocks' byte histograms, the tile counters, the active mask and the resolved count.
+// Start: clear the blocks' byte and digit histograms, the tile counters, the active mask and the resolved count.
 __global__ void k_lsd_begin(FwdArgs a) {
     Ctl *c = a.ctl;
     const u64 nh = (u64)a.B * 256;
     for (u64 i = (u64)blockIdx.x * blockDim.x + threadIdx.x; i < nh; i += (u64)gridDim.x * blockDim.x) a.lhist[i] = 0;
+    const u64 nb = lsd_coded(a) ? (u64)a.B * (NSLOT * 256 / 4) : 0;  // (raw keys: the digit bases are written whole)
+    uint4 *base4 = reinterpret_cast<uint4 *>(a.lbase);
+    for (u64 i = (u64)blockIdx.x * blockDim.x + threadIdx.x; i < nb; i += (u64)gridDim.x * blockDim.x)
+        base4[i] = make_uint4(0, 0, 0, 0);
     if (blockIdx.x == 0) {
         if (threadIdx.x < NSLOT) a.ltile[threadIdx.x] = 0;
         if (threadIdx.x == 0) {
@@ -107,12 +186,14 @@ __global__ void k_lsd_begin(FwdArgs a) {
             // whole rank buffer
             c->cnt[L_R0 + c->rpar] = a.idn;
             c->lsd_act = 0;
+            // coded keys: the segmentation takes the minimum over the groups that survive
+            c->h0 = lsd_coded(a) ? 0xFFFFFFFFu : a.lsd_bytes;
             c->m = a.blk[a.B - 1].soff + a.blk[a.B - 1].n;
         }
     }
 }
 
-// Each block's byte histogram, from which every pass's digit counts follow, and row 0 of its L column. CTA c takes a
+// Each block's byte histogram, from which its code follows, and row 0 of its L column. CTA c takes a
 // contiguous run of sort tiles and adds its shared histogram into a block's row when the run leaves it.
 __global__ void __launch_bounds__(TPB) k_lsd_key0(FwdArgs a) {
     __shared__ u32 hs[256];
@@ -145,7 +226,184 @@ __global__ void __launch_bounds__(TPB) k_lsd_key0(FwdArgs a) {
     if (cur != ~0u && hs[threadIdx.x]) atomicAdd(&a.lhist[(u64)cur * 256 + threadIdx.x], hs[threadIdx.x]);
 }
 
-// Digit bases of every pass and the active slots (256 threads per CTA, thread = digit value, CTAs over blocks).
+// The code of every block (CTAs over blocks, 256 threads, thread = byte value). The bytes that occur, in order, are
+// split again and again at the weight midpoint (the cut nearest to half of the interval's count, kept within what the
+// remaining levels can hold); a byte's codeword is its path. Every thread walks its own path over the cumulative
+// counts in shared memory: at most CODE_MAX levels of a binary search.
+__global__ void __launch_bounds__(TPB) k_lsd_code(FwdArgs a) {
+    __shared__ u32 C[257];
+    __shared__ u32 ws[TPB / 32 + 1];
+    __shared__ u32 len0;
+    const u32 x = threadIdx.x;
+    for (u32 b = blockIdx.x; b < a.B; b += gridDim.x) {
+        const u32 h = a.lhist[(u64)b * 256 + x];
+        u32 ns, n;
+        const u32 idx = block_excl_sum<TPB>(h != 0, ws, &ns);  // the byte's index among those that occur
+        const u32 before = block_excl_sum<TPB>(h, ws, &n);
+        if (h) C[idx] = before;
+        if (x == 0) C[ns] = n;
+        __syncthreads();
+        u32 code = 0, len = 0;
+        if (h) {
+            u32 lo = 0, hi = ns;
+            while (hi - lo > 1) {
+                const u32 half = 1u << (CODE_MAX - len - 1);
+                const u32 c0 = C[lo], c1 = C[hi], mid = c0 + (c1 - c0) / 2;
+                u32 l = lo + 1, r = hi - 1;  // the first cut in (lo, hi) at or past the midpoint (hi - 1 if none)
+                while (l < r) {
+                    const u32 m = (l + r) >> 1;
+                    if (C[m] >= mid) r = m; else l = m + 1;
+                }
+                if (l > lo + 1 && C[l] > mid && mid - C[l - 1] < C[l] - mid) l--;
+                if (l - lo > half) l = lo + half;
+                if (hi - l > half) l = hi - half;
+                code <<= 1;
+                if (idx < l) hi = l; else { lo = l; code |= 1; }
+                len++;
+            }
+            if (len == 0) len = 1;  // a block of one byte value
+            if (idx == 0) { len0 = len; a.ctab[(u64)b * CODE_ROW + CODE_MIN] = x; }
+        } else {
+            len = 1;  // not in the block; any length keeps the readers' loops finite
+        }
+        a.ctab[(u64)b * CODE_ROW + x] = code << (32 - len) | len;
+        __syncthreads();
+        if (x == 0) a.ctab[(u64)b * CODE_ROW + CODE_PAD] = len0;
+        __syncthreads();
+    }
+}
+
+// The keys of all suffixes in text order: each thread encodes 16 consecutive positions from right to left (the key at
+// a position is its codeword followed by the key of the next position, so after the first, encoded from the text
+// behind the run, each costs a table look-up and G funnel shifts; the codeword ends are carried the same way and
+// counted). Counts every key byte of its block (the digit histograms of all passes). CTA c takes a contiguous run of
+// sort tiles and adds its shared histograms into the block's rows when the run leaves it.
+struct KeySmem {
+    static constexpr int G = 2;  // key groups
+    u32 hist[4 * G][256];
+    u32 key[G][LSD_TILE + LSD_TILE / 16];  // padded: a thread's 16 keys are consecutive
+    u32 whole[LSD_TILE / 4];
+    u32 tab[CODE_ROW];
+};
+__global__ void __launch_bounds__(TPB) k_lsd_keys(FwdArgs a) {
+    __shared__ KeySmem S;
+    constexpr int G = KeySmem::G;
+    static_assert(LSD_IPT == 16, "a thread encodes 16 consecutive positions");
+    const u32 nt = a.ctl->lsd_tiles;
+    const u32 per = (nt + gridDim.x - 1) / gridDim.x;
+    const u32 t0 = blockIdx.x * per, t1 = min(nt, t0 + per);
+    if (t0 >= t1) return;
+    const u32 tid = threadIdx.x, lane = lane_id();
+    for (u32 i = tid; i < 4 * G * 256; i += TPB) (&S.hist[0][0])[i] = 0;
+    u32 cur = ~0u;  // block whose counts hist holds
+    auto flush = [&]() {
+        for (u32 i = tid; i < 4 * G * 256; i += TPB) {
+            const u32 v = (&S.hist[0][0])[i];
+            if (v) {
+                atomicAdd(&a.lbase[((u64)cur * NSLOT + (15 - (i >> 8))) * 256 + (i & 255)], v);
+                (&S.hist[0][0])[i] = 0;
+            }
+        }
+    };
+    for (u32 t = t0; t < t1; t++) {
+        const LsdTile tl = lsd_tile(a, t);
+        __syncthreads();
+        if (tl.b != cur) {
+            if (cur != ~0u) flush();
+            cur = tl.b;
+            for (u32 i = tid; i < CODE_ROW; i += TPB) S.tab[i] = a.ctab[(u64)tl.b * CODE_ROW + i];
+            __syncthreads();
+        }
+        const BlockInfo bi = a.blk[tl.b];
+        const u64 end = (u64)bi.off + bi.n;
+        const u32 x0 = tid * 16;
+        const u64 q0 = (u64)bi.off + (tl.base - bi.soff) + x0;
+        u32 k[G], m[G], wh[4] = {0, 0, 0, 0};
+#pragma unroll
+        for (int g = 0; g < G; g++) k[g] = m[g] = 0;
+        Text16 w = {};
+        if (x0 < tl.cnt) {  // (the run's first position lies in the block)
+            w = text16(a.T, q0, end);
+            lsd_encode<G>(a.T, S.tab, q0 + 16, end, k, m);
+        }
+#pragma unroll
+        for (int j = 15; j >= 0; j--) {
+            const u32 x = x0 + j;
+            const bool ok = x < tl.cnt;
+            // (symbols past the end of the block: the run's keys start from the end's zeros and its pad codewords)
+            if (ok) {
+                const u32 e = S.tab[(u32)((j < 8 ? w.w : w.w2) >> (8 * (j & 7))) & 0xFFu];
+                u32 d = 0;
+#pragma unroll
+                for (int g = G - 1; g > 0; g--) {
+                    k[g] = __funnelshift_r(k[g], k[g - 1], e);  // (count modulo 32)
+                    m[g] = __funnelshift_r(m[g], m[g - 1], e);
+                }
+                k[0] = __funnelshift_r(k[0], 0u, e) | (e & CODE_BITS);
+                m[0] = __funnelshift_r(m[0], 0u, e) | 1u << (32 - (e & 31u));
+#pragma unroll
+                for (int g = 0; g < G; g++) {
+                    S.key[g][x + (x >> 4)] = k[g];
+                    d += __popc(m[g]);
+                }
+                wh[j >> 2] |= d << (8 * (j & 3));  // at most 32 G <= 128
+            }
+#pragma unroll
+            for (int g = 0; g < G; g++) {
+                // runs of one key (padding, repeated records) would serialise 32 atomics on one counter
+                const u32 lead = __shfl_sync(0xffffffffu, k[g], 0);
+                const bool same = __all_sync(0xffffffffu, ok && k[g] == lead);
+                if (same ? lane == 0 : ok) {
+                    const u32 add = same ? 32u : 1u;
+#pragma unroll
+                    for (int b = 0; b < 4; b++) atomicAdd(&S.hist[4 * g + b][(k[g] >> (24 - 8 * b)) & 0xFFu], add);
+                }
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < 4; i++) S.whole[tid * 4 + i] = wh[i];
+        __syncthreads();
+#pragma unroll
+        for (int g = 0; g < G; g++) {
+            u32 *out = lsd_keys_of(a, g) + tl.base;
+            for (u32 x = tid; x < tl.cnt; x += TPB) out[x] = S.key[g][x + (x >> 4)];
+        }
+        u8 *out = lsd_whole_of(a) + tl.base;
+        for (u32 x = tid; x < tl.cnt; x += TPB) out[x] = reinterpret_cast<const u8 *>(S.whole)[x];
+    }
+    __syncthreads();
+    flush();
+}
+
+// Coded keys: digit bases of every pass and the active slots (CTAs over blocks, one warp per slot, eight digits per lane): the
+// exclusive scan of a block's digit counts plus the block's soff is the pass's first position of every digit (lbase
+// row (block, slot), in place of the counts). A slot runs when its key byte takes two or more values within some
+// block (slots 16 - W..15 only).
+__global__ void __launch_bounds__(TPB) k_lsd_base(FwdArgs a) {
+    const int first = 16 - (int)a.lsd_bytes;
+    for (u32 b = blockIdx.x; b < a.B; b += gridDim.x) {
+        const u32 n = a.blk[b].n, soff = a.blk[b].soff;
+        for (int slot = first + (int)warp_id(); slot < NSLOT; slot += TPB / 32) {
+            uint4 *row = reinterpret_cast<uint4 *>(a.lbase + ((u64)b * NSLOT + slot) * 256) + 2 * lane_id();
+            const uint4 u = row[0], v = row[1];
+            const u32 d[8] = {u.x, u.y, u.z, u.w, v.x, v.y, v.z, v.w};
+            u32 sum = 0;
+            bool vary = false;
+#pragma unroll
+            for (int i = 0; i < 8; i++) { sum += d[i]; vary = vary || (d[i] != 0 && d[i] != n); }
+            u32 run = soff + warp_incl_sum(sum) - sum;
+            u32 o[8];
+#pragma unroll
+            for (int i = 0; i < 8; i++) { o[i] = run; run += d[i]; }
+            row[0] = make_uint4(o[0], o[1], o[2], o[3]);
+            row[1] = make_uint4(o[4], o[5], o[6], o[7]);
+            if (__any_sync(0xffffffffu, vary) && lane_id() == 0 && !((a.ctl->lsd_act >> slot) & 1))
+                atomicOr(&a.ctl->lsd_act, 1u << slot);
+        }
+    }
+}
+
+// Raw keys: digit bases of every pass and the active slots (256 threads per CTA, thread = digit value, CTAs over blocks).
 // Suffix i of a block of n bytes has key byte d = T[i + d] when i + d < n, else 0, so the counts of key byte d are
 // the block's byte counts minus those of its first min(d, n) bytes, plus min(d, n) zeros; their exclusive scan plus
 // the block's soff gives the pass's first position of every digit (lbase row (block, slot), slot = 15 - d). A slot
@@ -203,7 +461,7 @@ struct LsdSmem {
 // look back over the block's earlier tiles for the offsets (bounded spin), stage the tile in shared memory in digit
 // order and write it out in runs. FULL: the tile holds LSD_TILE suffixes (every tile but a block's last), so no
 // element needs a bounds check.
-template <bool FULL>
+template <bool CODED, bool FULL>
 __device__ __forceinline__ void lsd_pass_tile(const FwdArgs &a, LsdSmem &S, int slot, u32 act, u64 epoch, u32 tile,
                                               const LsdTile &tl) {
     const u32 lower = act & ((1u << slot) - 1), higher = act & ~((2u << slot) - 1);
@@ -219,16 +477,16 @@ __device__ __forceinline__ void lsd_pass_tile(const FwdArgs &a, LsdSmem &S, int 
     u32 v[LSD_IPT], rr[LSD_IPT / 2], k[LSD_IPT];
     const u32 dsh = 8 * (slot & 3);  // byte 15 - slot of the prefix within the key group
     if (!lower) {
-        // the first pass: the tile's suffixes are still in text order, ids and keys come from the text
+        // the first pass: the suffixes are still in text order, as k_lsd_keys wrote their keys
         const BlockInfo bi = a.blk[tl.b];
-        const u32 id0 = bi.off + (base - bi.soff);
+        const u32 id0 = bi.off + (base - bi.soff), g = lsd_slot_group(slot);
         const u64 end = (u64)bi.off + bi.n;
-        const u32 g = lsd_slot_group(slot);
+        const u32 *keys = CODED ? lsd_keys_of(a, g) : nullptr;
 #pragma unroll
         for (int j = 0; j < LSD_IPT; j++) {
             const u32 x = warp * (32 * LSD_IPT) + j * 32 + lane;
             v[j] = id0 + x;
-            k[j] = (FULL || x < cnt) ? lsd_group(a.T, id0 + x, g, end) : 0u;
+            k[j] = !(FULL || x < cnt) ? 0u : CODED ? __ldcs(keys + base + x) : lsd_raw_group(a.T, id0 + x, g, end);
         }
     } else {
 #pragma unroll
@@ -313,14 +571,14 @@ __device__ __forceinline__ void lsd_pass_tile(const FwdArgs &a, LsdSmem &S, int 
         atomicExch((unsigned long long *)st, epoch | ST_PRE | (u64)(excl + tot));
     }
     S.gbase[tid] = dbase + excl - dstart;
+    const u32 g = lsd_slot_group(slot);
+    // the key the next pass reads: this group's (carried), the next group's (gathered) or none
+    const int gn = higher ? (int)lsd_slot_group(__ffs(higher) - 1) : -1;
     __syncthreads();
     unsigned long long *iout = a.lit[par ^ 1];
     const BlockInfo bi = a.blk[tl.b];
     const u32 bend = bi.soff + bi.n;  // bound of the checked build's write checks
     (void)bend;
-    // the key the next pass reads: this group's (carried), the next group's (gathered from the text) or none
-    const u32 g = lsd_slot_group(slot);
-    const int gn = higher ? (int)lsd_slot_group(__ffs(higher) - 1) : -1;
     if (gn == (int)g) {
         for (u32 i = tid; i < cnt; i += TPB) {
             const unsigned long long it = S.item[i];
@@ -329,21 +587,23 @@ __device__ __forceinline__ void lsd_pass_tile(const FwdArgs &a, LsdSmem &S, int 
         }
     } else if (gn >= 0) {
         const u64 end = (u64)bi.off + bi.n;
-        constexpr int WB = 4;  // gathers in flight per thread
+        const u32 *keys = CODED ? lsd_keys_of(a, (u32)gn) : nullptr;
+        const u32 dense = bi.soff - bi.off;  // (modulo 2^32: a batch with gaps has off > soff)
+        constexpr int WB = CODED ? 8 : 4;  // gathers in flight per thread
         for (u32 i0 = tid; i0 < cnt; i0 += WB * TPB) {
-            u32 id[WB], kk[WB], dst[WB];
+            u32 id[WB], dst[WB], kk[WB];
 #pragma unroll
             for (int q = 0; q < WB; q++) {
                 const u32 i = i0 + q * TPB;
-                const bool ok = i < cnt;
+                const bool ok = FULL || i < cnt;
                 const unsigned long long it = ok ? S.item[i] : 0ull;
                 id[q] = (u32)it;
                 dst[q] = ok ? S.gbase[((u32)(it >> 32) >> dsh) & 0xFFu] + i : 0u;
-                kk[q] = ok ? lsd_group(a.T, id[q], (u32)gn, end) : 0u;
+                kk[q] = !ok ? 0u : CODED ? __ldg(keys + (u32)(dense + id[q])) : lsd_raw_group(a.T, id[q], (u32)gn, end);
             }
 #pragma unroll
             for (int q = 0; q < WB; q++) {
-                if (i0 + q * TPB < cnt && KGB_OK(dst[q] < bend, &a.ctl->err, E_LIST)) {
+                if ((FULL || i0 + q * TPB < cnt) && KGB_OK(dst[q] < bend, &a.ctl->err, E_LIST)) {
                     __stcs(iout + dst[q], (unsigned long long)kk[q] << 32 | id[q]);
                 }
             }
@@ -360,6 +620,7 @@ __device__ __forceinline__ void lsd_pass_tile(const FwdArgs &a, LsdSmem &S, int 
 
 // One LSD pass over digit `slot` (skipped when that key byte is constant within every block): each CTA takes the
 // next sort tile in order.
+template <bool CODED>
 __global__ void __launch_bounds__(TPB, 3) k_lsd_pass(FwdArgs a, int slot) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     LsdSmem &S = *reinterpret_cast<LsdSmem *>(smem_raw);
@@ -375,8 +636,8 @@ __global__ void __launch_bounds__(TPB, 3) k_lsd_pass(FwdArgs a, int slot) {
     const u32 tile = S.tile;
     if (tile >= ntiles) return;
     const LsdTile tl = lsd_tile(a, tile);
-    if (tl.cnt == (u32)LSD_TILE) lsd_pass_tile<true>(a, S, slot, act, epoch, tile, tl);
-    else lsd_pass_tile<false>(a, S, slot, act, epoch, tile, tl);
+    if (tl.cnt == (u32)LSD_TILE) lsd_pass_tile<CODED, true>(a, S, slot, act, epoch, tile, tl);
+    else lsd_pass_tile<CODED, false>(a, S, slot, act, epoch, tile, tl);
 }
 
 // ---- segmentation of the sorted keys
@@ -389,6 +650,7 @@ __device__ __forceinline__ u32 lsd_final_par(const Ctl *c) { return __popc(activ
 struct SegBufs {
     const u32 *val;
     u32 *bits;          // start bitmask
+    u8 *dep;            // per position: the bytes its key holds whole (in a list that is empty in round 0)
     u32 *gbase, *gidx;  // per group start: list slot base, list index | GRP_LARGE (free value buffers)
     u32 *rk;            // per position: the round-0 rank, for the rank passes (the free half of the ids' item buffer)
     u32 m;
@@ -399,6 +661,7 @@ __device__ __forceinline__ SegBufs seg_bufs(const FwdArgs &a) {
     SegBufs v;
     v.val = a.lval[par];
     v.bits = a.segbits;
+    v.dep = reinterpret_cast<u8 *>(a.lists[L_S0].eid);
     v.gbase = a.lval[par ^ 1];
     v.gidx = a.lhi[par ^ 1];  // lval[q] and lhi[q] are the two halves of item buffer q
     v.rk = a.lhi[par];
@@ -415,41 +678,102 @@ __device__ __forceinline__ uint2 seg_chunk_blocks(const FwdArgs &a, u32 cb, u32 
     return make_uint2(lo, hi);
 }
 
-// Per tile: start bits and the tile's last group start (position 0 always starts a group, and so does every block's
-// first position).
-__global__ void __launch_bounds__(TPB) k_seg_count(FwdArgs a) {
+// Per tile: start bits and the tile's last group start. A position starts a group when it is its block's first or when
+// its suffix and the one before it differ in the bytes their keys hold whole (in their number, or in one of them): the
+// bits of a last codeword that the key cuts off do not count, so that a group has those bytes in common, and comparing
+// the text (which the L column's bytes are taken from here as well, coalesced) costs less than encoding it again.
+// Also per position the number of those bytes (at most DEPTH_MAX), and their minimum over the suffixes that start no
+// group (every group of two or more has one).
+template <bool CODED>
+__global__ void __launch_bounds__(TPB, 3) k_seg_count(FwdArgs a) {
     __shared__ u32 ws[TPB / 32];
     const SegBufs v = seg_bufs(a);
+    const u8 *whole = lsd_whole_of(a);
     const u32 ntiles = (v.m + SEG_TILE - 1) / SEG_TILE;
     const u32 lane = lane_id(), warp = warp_id();
-    // the prefix's second 8-byte word: its first W - 8 bytes (none for W = 8)
-    const u64 m2 = a.lsd_bytes >= 16 ? ~0ull : a.lsd_bytes == 12 ? 0xFFFFFFFF00000000ull : 0ull;
-    const bool two = m2 != 0;
+    u32 depth = 0xFFFFFFFFu;
     for (u32 t = blockIdx.x; t < ntiles; t += gridDim.x) {
         const u32 cb = t * SEG_TILE + warp * 32 * SEG_IPT;
         const uint2 br = cb < v.m ? seg_chunk_blocks(a, cb, v.m) : make_uint2(0u, 0u);
+        const BlockInfo bi0 = a.blk[br.x];
+        const u32 min0 = CODED ? a.ctab[(u64)br.x * CODE_ROW + CODE_MIN] : 0u;
+        // the suffix at the position before the step's first one (its block's: used where that position has the same)
+        u32 pid = cb > bi0.soff && cb < v.m ? v.val[cb - 1] : bi0.off, pd;
+        u64 pw, pw2;
+        {
+            const Text16 x = text16_padded(a.T, pid, (u64)bi0.off + bi0.n, min0);
+            pd = CODED ? whole[bi0.soff + (pid - bi0.off)] : a.lsd_bytes;
+            pw = x.w;
+            pw2 = x.w2;
+        }
         u32 last = 0;
-#pragma unroll 4
-        for (int j = 0; j < SEG_IPT; j++) {
-            const u32 p = cb + j * 32 + lane;
-            const bool ok = p < v.m;
-            const u32 b = ok ? (br.x == br.y ? br.x : blk_of_pos(a, p, br.x, br.y)) : 0u;
-            const BlockInfo bi = a.blk[b];
-            const u64 end = (u64)bi.off + bi.n;
-            // the prefix's two 8-byte words (the second cut to its first W - 8 bytes), from the text
-            const u32 id = ok ? v.val[p] : 0u;
-            u64 k = 0, k2 = 0;
-            if (ok) lsd_key16(a.T, id, end, two, k, k2);
-            k2 &= m2;
-            u64 kp = __shfl_up_sync(0xffffffffu, k, 1), k2p = __shfl_up_sync(0xffffffffu, k2, 1);
-            if (lane == 0 && ok && p > bi.soff) {  // the neighbour is in the same block
-                lsd_key16(a.T, v.val[p - 1], end, two, kp, k2p);
-                k2p &= m2;
+        constexpr int QB = 4;  // positions whose ids, text and counts are loaded at once
+#pragma unroll 1
+        for (int j0 = 0; j0 < SEG_IPT; j0 += QB) {
+            u32 id[QB], d[QB], b[QB];
+            Text16 tx[QB];
+#pragma unroll
+            for (int q = 0; q < QB; q++) {
+                const u32 p = cb + (j0 + q) * 32 + lane;
+                b[q] = p < v.m && br.x != br.y ? blk_of_pos(a, p, br.x, br.y) : br.x;
+                id[q] = p < v.m ? v.val[p] : bi0.off;
             }
-            const bool st = ok && (p == bi.soff || k != kp || k2 != k2p);
-            const u32 sb = __ballot_sync(0xffffffffu, st);
-            if (lane == 0 && cb + j * 32 < v.m) v.bits[(cb >> 5) + j] = sb;
-            if (st) last = p;
+#pragma unroll
+            for (int q = 0; q < QB; q++) {
+                BlockInfo bi = bi0;
+                u32 mn = min0;
+                if (br.x != br.y) { bi = a.blk[b[q]]; mn = CODED ? a.ctab[(u64)b[q] * CODE_ROW + CODE_MIN] : 0u; }
+                tx[q] = text16_padded(a.T, id[q], (u64)bi.off + bi.n, mn);
+                d[q] = CODED ? whole[bi.soff + (id[q] - bi.off)] : a.lsd_bytes;
+            }
+#pragma unroll
+            for (int q = 0; q < QB; q++) {
+                const u32 p = cb + (j0 + q) * 32 + lane;
+                const bool ok = p < v.m;
+                BlockInfo bi = bi0;
+                if (br.x != br.y) bi = a.blk[b[q]];
+                const u64 end = (u64)bi.off + bi.n;
+                // the neighbour's text, count and id: the lane below's, for lane 0 the last lane's of the step before
+                const u32 below = (lane + 31) & 31;
+                u64 nw = __shfl_sync(0xffffffffu, tx[q].w, below), nw2 = __shfl_sync(0xffffffffu, tx[q].w2, below);
+                u32 nd = d[q], nid = __shfl_sync(0xffffffffu, id[q], below);
+                if (CODED) nd = __shfl_sync(0xffffffffu, d[q], below);
+                if (lane == 0) {
+                    const u64 cw = nw, cw2 = nw2;
+                    const u32 cd = nd, cid = nid;
+                    nw = pw; nw2 = pw2; nd = pd; nid = pid;
+                    pw = cw; pw2 = cw2; pd = cd; pid = cid;
+                }
+                const u32 D = d[q];  // at least 5: CODE_MAX-bit codewords in 64 bits
+                bool eq = ok && p != bi.soff && nd == D;
+                const u64 x = tx[q].w ^ nw, x2 = tx[q].w2 ^ nw2;
+                eq = eq && (D >= 8 ? x == 0 : x << (8 * (8 - D)) == 0);
+                eq = eq && (D <= 8 || (D >= 16 ? x2 == 0 : x2 << (8 * (16 - D)) == 0));
+                // short codewords: the bytes past the first 16
+                for (u32 o = 16; CODED && __any_sync(0xffffffffu, eq && D > o); o += 16) {
+                    if (eq && D > o) {
+                        const u32 mn = a.ctab[(u64)b[q] * CODE_ROW + CODE_MIN];
+                        const Text16 y = text16_padded(a.T, (u64)id[q] + o, end, mn);
+                        const Text16 z = text16_padded(a.T, (u64)nid + o, end, mn);
+                        const u64 u = y.w ^ z.w, u2 = y.w2 ^ z.w2;
+                        const u32 r = D - o;
+                        eq = r >= 8 ? u == 0 : u << (8 * (8 - r)) == 0;
+                        eq = eq && (r <= 8 || (r >= 16 ? u2 == 0 : u2 << (8 * (16 - r)) == 0));
+                    }
+                }
+                const bool st = ok && !eq;
+                const u32 sb = __ballot_sync(0xffffffffu, st);
+                if (lane == 0 && ok) v.bits[(cb >> 5) + j0 + q] = sb;
+                if (ok) {
+                    if (CODED) v.dep[p] = (u8)min(D, DEPTH_MAX);
+                    // the L column of the sorted order so far: final for groups of one, overwritten for the others
+                    const u8 c = id[q] == bi.off ? (u8)0 : tx[q].has_before ? tx[q].before : __ldg(a.T + id[q] - 1);
+                    KGB_GUARD(p >= bi.soff && p - bi.soff < bi.n, &a.ctl->err, E_RANK)
+                    a.L[(u64)bi.off + b[q] + (p - bi.soff) + 1] = c;
+                }
+                if (st) last = p;
+                if (CODED && eq) depth = min(depth, D);
+            }
         }
 #pragma unroll
         for (int o = 16; o; o >>= 1) last = max(last, __shfl_xor_sync(0xffffffffu, last, o));
@@ -462,6 +786,9 @@ __global__ void __launch_bounds__(TPB) k_seg_count(FwdArgs a) {
         }
         __syncthreads();
     }
+    if (!CODED) return;
+    depth = __reduce_min_sync(0xffffffffu, depth);
+    if (lane == 0 && depth != 0xFFFFFFFFu && depth < *(volatile u32 *)&a.ctl->h0) atomicMin(&a.ctl->h0, depth);
 }
 
 // Exclusive max-scan of the tiles' last starts (one CTA): the start of the group open at each tile's first position.
@@ -548,11 +875,10 @@ __device__ __forceinline__ u64 block_excl_sum64(u64 v, u64 *ws, u64 *total) {
     return before + inc - v;
 }
 
-// Emit, part 1 (group ends): groups of one resolve (rank unless k_seg_rank writes the ranks, L column); every other
-// group takes its slots in the next tiny-group list
-// (<= GTINY), medium-group list (<= GMED), small-group list (<= SMAX) or large-group list, writes its descriptor (and
-// tile-map entries), and records its slot base and index at its first position for part 2. Slots are allocated once
-// per tile (a count pass, a block scan, one atomic per list).
+// Emit, part 1 (group ends): groups of one resolve (rank unless k_seg_rank writes the ranks); every other group takes
+// its slots in the next tiny-group list (<= GTINY), medium-group list (<= GMED), small-group list (<= SMAX) or
+// large-group list, writes its descriptor (and tile-map entries), and records its slot base and index at its first
+// position for part 2. Slots are allocated once per tile (a count pass, a block scan, one atomic per list).
 __global__ void __launch_bounds__(TPB) k_seg_emit1(FwdArgs a) {
     __shared__ u32 wl[TPB / 32];
     __shared__ u64 ws[4][TPB / 32];
@@ -616,12 +942,13 @@ __global__ void __launch_bounds__(TPB) k_seg_emit1(FwdArgs a) {
                 pv[q] = p; gfv[q] = gf;
                 if (ok && en) live |= 1u << q;
             }
-            u32 bv[QB], idv[QB];
+            u32 bv[QB], idv[QB];  // idv: the id of a finished suffix (a group of one), else the group's shared characters
+            const bool ids = !a.rank_passes || a.SA;
 #pragma unroll
             for (int q = 0; q < QB; q++) {
                 if (!((live >> q) & 1)) continue;
                 bv[q] = ch.blo == ch.bhi ? ch.blo : blk_of_pos(a, pv[q], ch.blo, ch.bhi);
-                idv[q] = pv[q] == gfv[q] ? __ldg(v.val + pv[q]) : 0u;  // ids of finished suffixes (groups of one)
+                idv[q] = pv[q] != gfv[q] ? (lsd_coded(a) ? (u32)__ldg(v.dep + pv[q]) : 0u) : ids ? __ldg(v.val + pv[q]) : 0u;
             }
 #pragma unroll
             for (int q = 0; q < QB; q++) {
@@ -631,11 +958,11 @@ __global__ void __launch_bounds__(TPB) k_seg_emit1(FwdArgs a) {
                 const u32 b = bv[q];
                 const u32 head = gf - a.blk[b].soff;
                 if (len == 1) {
-                    resolve_round0(a, a.rank_passes ? nullptr : a.isa[rpar ^ 1], idv[q], head, b);
+                    if (ids) resolve_round0(a, a.rank_passes ? nullptr : a.isa[rpar ^ 1], idv[q], head, b);
                     continue;
                 }
                 Seg g;
-                g.len = len; g.head = head; g.bd = b;
+                g.len = len; g.head = head; g.bd = b | idv[q] << DEPTH_SHIFT;
                 if (len <= GTINY) {
                     g.start = te;
                     KGB_GUARD(tidx < a.cap_segt && (u64)te + len <= a.cap_n, &c->err, E_SEG) {
