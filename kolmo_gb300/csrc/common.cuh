@@ -65,6 +65,51 @@ __device__ __forceinline__ u32 warp_sum(u32 v) {
     return v;
 }
 
+// Stable ranks by digit (< 256) within a warp, Q elements per lane at once (element q of every lane before element
+// q + 1 of any): rank[q] = elements of the same digit counted in cnt before + those of this call that come first. `cnt`
+// holds the warp's 256 counters and is advanced; `mask` is 256 Q words of the warp's own shared memory, all zero before
+// and after. Elements past the end carry digit 256 (CHECK) and take no rank.
+//
+// The lanes that share a digit are found from two pivots (lane 0's digit and the first other one: a shuffle and a
+// ballot each) and, for the rest, by collecting lane bits with one shared-memory atomic. __match_any_sync takes two
+// cycles per SM and distinct digit: 59 for 32 lanes of evenly spread digits, 27 for letters of text, 5 for four
+// values; the atomics alone take 10, 11 and 14, but 36 where one digit fills the warp; with the pivots it is 12, 12 and
+// 14, and 8 there. Q elements in flight hide the atomics' latency; one lane per digit advances the counter for all
+// (atomics of one warp to shared memory take effect in program order).
+template <int Q, bool CHECK>
+__device__ __forceinline__ void warp_rank(u32 *mask, u32 *cnt, const u32 (&d)[Q], u32 (&rank)[Q]) {
+    const u32 all = 0xffffffffu, bit = 1u << lane_id();
+    u32 peers[Q];
+    bool rest[Q];
+#pragma unroll
+    for (int q = 0; q < Q; q++) {
+        const u32 d0 = __shfl_sync(all, d[q], 0);
+        const u32 b0 = __ballot_sync(all, d[q] == d0);
+        const u32 d1 = __shfl_sync(all, d[q], __ffs(~b0) - 1);  // (every lane holds d0: any lane will do)
+        const u32 b1 = __ballot_sync(all, d[q] == d1);
+        peers[q] = d[q] == d0 ? b0 : b1;
+        rest[q] = d[q] != d0 && d[q] != d1 && !(CHECK && d[q] > 255);
+        if (rest[q]) atomicOr(mask + 256 * q + d[q], bit);
+    }
+    __syncwarp();
+#pragma unroll
+    for (int q = 0; q < Q; q++)
+        if (rest[q]) peers[q] = *(volatile u32 *)(mask + 256 * q + d[q]);
+    __syncwarp();
+#pragma unroll
+    for (int q = 0; q < Q; q++) {
+        rank[q] = 0;
+        if ((peers[q] & (bit - 1)) == 0 && !(CHECK && d[q] > 255)) {  // the digit's first lane
+            rank[q] = atomicAdd(cnt + d[q], (u32)__popc(peers[q]));
+            if (rest[q]) mask[256 * q + d[q]] = 0;
+        }
+    }
+#pragma unroll
+    for (int q = 0; q < Q; q++)
+        rank[q] = __shfl_sync(all, rank[q], __ffs(peers[q]) - 1) + __popc(peers[q] & (bit - 1));
+    __syncwarp();
+}
+
 // Block-wide exclusive sum over NT threads (NT multiple of 32, <= 1024). `ws` needs NT/32 + 1 words of shared
 // memory. Returns the thread's exclusive prefix; *total receives the block sum. Contains __syncthreads().
 template <int NT>

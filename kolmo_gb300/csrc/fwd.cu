@@ -186,7 +186,7 @@ struct TileSmem {
     KeyT klo[TILE];
     u32 val[TILE];
     u16 khi[TILE];
-    u16 wcnt[TPB / 32][256];
+    u32 wcnt[TPB / 32][256];
     u32 lstart[TS + 1];
     u32 lhead[TS];
     u32 lblk[TS];
@@ -360,19 +360,23 @@ __global__ void __launch_bounds__(TPB, TileTraits<PREFIX, TILE>::MINB) k_tile_so
             const bool lo_part = digit < KB;
             const u32 sh = lo_part ? 8 * digit : 8 * (digit - KB);
             if (lo_part ? !((vary_lo >> sh) & 0xFF) : !((vary_hi >> sh) & 0xFF)) continue;
+            // (the digit masks borrow val, which the elements leave for registers before each digit)
+            constexpr int RQ = 2;
+            static_assert(sizeof(S.val) >= NW * 256 * RQ * 4, "mask words");
+            u32 *mask = S.val + warp * 256 * RQ;
             for (int i = tid; i < NW * 256; i += TPB) (&S.wcnt[0][0])[i] = 0;
+            for (int i = tid; i < NW * 256 * RQ; i += TPB) S.val[i] = 0;
             __syncthreads();
             u32 dg[IPT], rk[IPT];
 #pragma unroll
-            for (int j = 0; j < IPT; j++) {
-                const u32 d = lo_part ? (u32)(k[j] >> sh) & 0xFF : (hi[j] >> sh) & 0xFF;
-                dg[j] = d;
-                const u32 peers = __match_any_sync(0xffffffffu, d);
-                const u32 before = S.wcnt[warp][d];
-                rk[j] = before + __popc(peers & lanemask_lt());
-                __syncwarp();
-                if ((__ffs(peers) - 1) == (int)lane) S.wcnt[warp][d] = (u16)(before + __popc(peers));
-                __syncwarp();
+            for (int j = 0; j < IPT; j += RQ) {
+                u32 d[RQ], r[RQ];
+#pragma unroll
+                for (int q = 0; q < RQ; q++)
+                    dg[j + q] = d[q] = lo_part ? (u32)(k[j + q] >> sh) & 0xFF : (hi[j + q] >> sh) & 0xFF;
+                warp_rank<RQ, false>(mask, S.wcnt[warp], d, r);
+#pragma unroll
+                for (int q = 0; q < RQ; q++) rk[j + q] = r[q];
             }
             __syncthreads();
             {   // digit-major exclusive scan: thread tid owns digit tid
@@ -381,7 +385,7 @@ __global__ void __launch_bounds__(TPB, TileTraits<PREFIX, TILE>::MINB) k_tile_so
                 for (int w = 0; w < NW; w++) tot += S.wcnt[w][tid];
                 u32 run = block_excl_sum<TPB>(tot, S.ws, nullptr);
 #pragma unroll
-                for (int w = 0; w < NW; w++) { u32 cc = S.wcnt[w][tid]; S.wcnt[w][tid] = (u16)run; run += cc; }
+                for (int w = 0; w < NW; w++) { u32 cc = S.wcnt[w][tid]; S.wcnt[w][tid] = run; run += cc; }
             }
             __syncthreads();
 #pragma unroll
@@ -1483,8 +1487,9 @@ __global__ void __launch_bounds__(TPB) k_msd_hist(FwdArgs a) {
                 }
                 kk = ((u32)sel << 8) | d;
             }
-            const u32 peers = __match_any_sync(0xffffffffu, kk);
-            if (valid && (__ffs(peers) - 1) == (int)lane) atomicAdd(&(&hs[0][0])[kk], __popc(peers));
+            // one atomic for the elements that share lane 0's digit (a group's keys mostly share one), one for each other
+            const u32 k0 = __shfl_sync(0xffffffffu, kk, 0), b0 = __ballot_sync(0xffffffffu, kk == k0);
+            if (valid && (kk != k0 || lane == 0)) atomicAdd(&(&hs[0][0])[kk], kk == k0 ? (u32)__popc(b0) : 1u);
         }
         if (PREFIX) {
 #pragma unroll
@@ -1662,6 +1667,7 @@ __global__ void __launch_bounds__(TPB) k_msd_scatter(FwdArgs a) {
                 const u32 d = msd_digit<PREFIX>(a, in, x, ids[j], sel ? m.g1 : m.g0, sel ? m.d1 : m.d0, &keys[j]);
                 kk[j] = ((u32)sel << 8) | d;
             }
+            // (a warp's elements fall into few buckets here, where __match_any_sync costs less than atomics)
             const u32 peers = __match_any_sync(0xffffffffu, kk[j]);
             const int leader = __ffs(peers) - 1;
             u32 old = 0;

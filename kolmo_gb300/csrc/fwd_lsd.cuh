@@ -33,11 +33,11 @@ constexpr u64 ST_AGG = 1ull << 30, ST_PRE = 2ull << 30, ST_VAL = (1ull << 30) - 
 constexpr u64 ST_EPOCH = 0xFFFFFFFF00000000ull;
 constexpr int LB_WIN = 8;  // look-back window (predecessor words read per step)
 
-// Which keys: the tuning table's choice per batch size, by measurement. Coded keys halve the passes but compare more in
-// the segmentation and leave slightly larger groups. Coded against the best raw width, all kernels of the call: 1 MiB
-// Markov block 0.31 ms against 0.44, 64 slices of 512 KiB prose 4.8 against 5.3, 64 mixed blocks (216 MB) 31.7 against
-// 33.9; on single blocks of prose over 32 MiB the deeper raw 16 bytes win (64 MiB: 15.5 against 16.1), because there
-// the rank rounds' gathers miss L2 and every active suffix they are left costs fifteen passes' worth.
+// Which keys: the tuning table's choice per batch size, by measurement. Coded keys halve the passes, compare more in the
+// segmentation and leave slightly larger groups. Forward call, coded against the best raw width: 1 MiB Markov block
+// 0.24 ms against 0.29, ACGT 0.24 and 0.28, log lines 0.52 and 0.52, prose 0.73 and 0.72; 16 MiB 1.73 and 2.24, 1.69 and
+// 2.24, 3.14 and 3.37, 3.68 and 3.85; mixed batch of 64 blocks (216 MB) 28.9 and 34.3. Between 32 and 128 MiB the table
+// keeps raw 16 bytes for the sake of prose (64 MiB: 15.5 against 15.7).
 __host__ __device__ __forceinline__ bool lsd_coded(const FwdArgs &a) { return a.lsd_bytes == 8; }
 __device__ __forceinline__ u32 active_slots(const Ctl *c) { return c->lsd_act; }  // bit s: slot s varies
 
@@ -449,9 +449,10 @@ __global__ void __launch_bounds__(TPB) k_lsd_ident(FwdArgs a) {
     }
 }
 
+constexpr int RANK_Q = 4;  // elements a lane ranks at once
 struct LsdSmem {
     unsigned long long item[LSD_TILE];
-    u16 wcnt[TPB / 32][256];
+    __align__(16) u32 wcnt[TPB / 32][256];
     u32 gbase[256];
     u32 ws[TPB / 32 + 1];
     u32 tile;
@@ -476,6 +477,7 @@ __device__ __forceinline__ void lsd_pass_tile(const FwdArgs &a, LsdSmem &S, int 
     // recomputed from the key where it is needed
     u32 v[LSD_IPT], rr[LSD_IPT / 2], k[LSD_IPT];
     const u32 dsh = 8 * (slot & 3);  // byte 15 - slot of the prefix within the key group
+    u32 *mask = reinterpret_cast<u32 *>(S.item) + warp * 256 * RANK_Q;  // (zeroed; the staging follows the ranking)
     if (!lower) {
         // the first pass: the suffixes are still in text order, as k_lsd_keys wrote their keys
         const BlockInfo bi = a.blk[tl.b];
@@ -498,17 +500,35 @@ __device__ __forceinline__ void lsd_pass_tile(const FwdArgs &a, LsdSmem &S, int 
             k[j] = (u32)(it >> 32);
         }
     }
+    // Coded keys spread over the digit values; raw text, sorted by what follows, has few distinct bytes in a warp, and
+    // __match_any_sync takes two cycles a distinct value (64 MiB of prose, 16 passes: 7.24 ms with it, 7.34 with
+    // warp_rank; 216 MB of mixed blocks, 8 passes over coded keys: 14.4 and 11.7).
+    if (CODED) {
 #pragma unroll
-    for (int j = 0; j < LSD_IPT; j++) {
-        const u32 x = warp * (32 * LSD_IPT) + j * 32 + lane;
-        const u32 d = (FULL || x < cnt) ? (k[j] >> dsh) & 0xFFu : 0x100u;  // 0x100: past the tile's end
-        const u32 peers = __match_any_sync(0xffffffffu, d);
-        const u32 before = (FULL || d < 256) ? S.wcnt[warp][d] : 0u;
-        const u32 r = before + __popc(peers & lanemask_lt());
-        if (j & 1) rr[j >> 1] |= r << 16; else rr[j >> 1] = r;
-        __syncwarp();
-        if ((FULL || d < 256) && (__ffs(peers) - 1) == (int)lane) S.wcnt[warp][d] = (u16)(before + __popc(peers));
-        __syncwarp();
+        for (int j0 = 0; j0 < LSD_IPT; j0 += RANK_Q) {
+            u32 d[RANK_Q], r[RANK_Q];
+#pragma unroll
+            for (int q = 0; q < RANK_Q; q++) {
+                const u32 x = warp * (32 * LSD_IPT) + (j0 + q) * 32 + lane;
+                d[q] = (FULL || x < cnt) ? (k[j0 + q] >> dsh) & 0xFFu : 0x100u;  // 0x100: past the tile's end
+            }
+            warp_rank<RANK_Q, !FULL>(mask, S.wcnt[warp], d, r);
+#pragma unroll
+            for (int q = 0; q < RANK_Q; q += 2) rr[(j0 + q) >> 1] = r[q] | r[q + 1] << 16;
+        }
+    } else {
+#pragma unroll
+        for (int j = 0; j < LSD_IPT; j++) {
+            const u32 x = warp * (32 * LSD_IPT) + j * 32 + lane;
+            const u32 d = (FULL || x < cnt) ? (k[j] >> dsh) & 0xFFu : 0x100u;  // 0x100: past the tile's end
+            const u32 peers = __match_any_sync(0xffffffffu, d);
+            const u32 before = (FULL || d < 256) ? S.wcnt[warp][d] : 0u;
+            const u32 r = before + __popc(peers & lanemask_lt());
+            if (j & 1) rr[j >> 1] |= r << 16; else rr[j >> 1] = r;
+            __syncwarp();
+            if ((FULL || d < 256) && (__ffs(peers) - 1) == (int)lane) S.wcnt[warp][d] = before + __popc(peers);
+            __syncwarp();
+        }
     }
     __syncthreads();
     // thread tid owns digit tid: tile count, publish, local start, look back
@@ -522,7 +542,7 @@ __device__ __forceinline__ void lsd_pass_tile(const FwdArgs &a, LsdSmem &S, int 
     {
         u32 run = dstart;
 #pragma unroll
-        for (int w = 0; w < TPB / 32; w++) { const u32 cc = S.wcnt[w][tid]; S.wcnt[w][tid] = (u16)run; run += cc; }
+        for (int w = 0; w < TPB / 32; w++) { const u32 cc = S.wcnt[w][tid]; S.wcnt[w][tid] = run; run += cc; }
     }
     __syncthreads();
     // stage in digit order (tile-local offsets only: the items leave registers before the look-back)
@@ -631,7 +651,12 @@ __global__ void __launch_bounds__(TPB, 3) k_lsd_pass(FwdArgs a, int slot) {
     const u64 epoch = (u64)((c->seq << 5) | (u32)slot) << 32;
     const u32 tid = threadIdx.x;
     if (tid == 0) S.tile = atomicAdd(&a.ltile[slot], 1u);
-    for (int i = tid; i < (TPB / 32) * 256; i += TPB) (&S.wcnt[0][0])[i] = 0;
+    {  // the ranking's counters and digit masks (the masks borrow the staging area)
+        static_assert(sizeof(S.item) == (TPB / 32) * 256 * RANK_Q * 4 && sizeof(S.wcnt) % (16 * TPB) == 0, "");
+        const uint4 z = make_uint4(0, 0, 0, 0);
+        for (u32 i = tid; i < sizeof(S.wcnt) / 16; i += TPB) reinterpret_cast<uint4 *>(&S.wcnt[0][0])[i] = z;
+        for (u32 i = tid; CODED && i < sizeof(S.item) / 16; i += TPB) reinterpret_cast<uint4 *>(S.item)[i] = z;
+    }
     __syncthreads();
     const u32 tile = S.tile;
     if (tile >= ntiles) return;

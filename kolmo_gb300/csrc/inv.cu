@@ -96,8 +96,12 @@ __global__ void __launch_bounds__(ITPB) k_inv_chunkhist(InvArgs a) {
         for (u32 i0 = 0; i0 < cnt; i0 += ITPB) {
             const u32 i = i0 + threadIdx.x;
             const u32 c = i < cnt ? (u32)src[i] : 0x100u;
-            const u32 peers = __match_any_sync(0xffffffffu, c);
-            if (c < 256 && (__ffs(peers) - 1) == (int)lane) atomicAdd(&h[c], __popc(peers));
+            // (runs of one byte would serialise 32 atomics on one counter)
+            if (__all_sync(0xffffffffu, c == __shfl_sync(0xffffffffu, c, 0))) {
+                if (c < 256 && lane == 0) atomicAdd(&h[c], 32u);
+            } else if (c < 256) {
+                atomicAdd(&h[c], 1u);
+            }
         }
         __syncthreads();
         a.csum[q * 256 + threadIdx.x] = h[threadIdx.x];
@@ -147,12 +151,15 @@ __global__ void __launch_bounds__(ITPB) k_inv_chunkscan(InvArgs a) {
 
 // Stable scatter, one CTA per chunk walking its tiles in order: psi[C[c] + occurrences of c before row q] = q,
 // with the mark flag of q.
-__global__ void __launch_bounds__(ITPB) k_inv_scatter(InvArgs a) {
+__global__ void __launch_bounds__(ITPB, 3) k_inv_scatter(InvArgs a) {
     constexpr int NW = ITPB / 32, IPT = ITILE / ITPB, WS = 32 * IPT;
-    __shared__ u16 wc[NW][256];
+    constexpr int RQ = 4;  // elements a lane ranks at once
+    __shared__ u32 wc[NW][256];
+    __shared__ u32 mask[NW][256 * RQ];  // (zero between uses)
     __shared__ u32 woff[NW][256];
     __shared__ u32 run_s[256];
     const u32 lane = lane_id(), warp = warp_id();
+    for (int i = threadIdx.x; i < NW * 256 * RQ; i += ITPB) (&mask[0][0])[i] = 0;
     for (u64 q = blockIdx.x; q < a.nchunk_all; q += gridDim.x) {
         const u32 b = a.cblk[q];
         const InvBlock B = a.blk[b];
@@ -169,14 +176,16 @@ __global__ void __launch_bounds__(ITPB) k_inv_scatter(InvArgs a) {
 #pragma unroll
             for (int j = 0; j < IPT; j++) {
                 const u32 x = warp * WS + j * 32 + lane;
-                const u32 c = x < cnt ? (u32)a.U[(u64)B.off + start + x] : 0x100u;
-                cs[j] = c;
-                const u32 peers = __match_any_sync(0xffffffffu, c);
-                const u32 before = c < 256 ? wc[warp][c] : 0u;
-                rk[j] = before + __popc(peers & lanemask_lt());
-                __syncwarp();
-                if (c < 256 && (__ffs(peers) - 1) == (int)lane) wc[warp][c] = (u16)(before + __popc(peers));
-                __syncwarp();
+                cs[j] = x < cnt ? (u32)a.U[(u64)B.off + start + x] : 0x100u;
+            }
+#pragma unroll
+            for (int j = 0; j < IPT; j += RQ) {
+                u32 c[RQ], r[RQ];
+#pragma unroll
+                for (int q = 0; q < RQ; q++) c[q] = cs[j + q];
+                warp_rank<RQ, true>(mask[warp], wc[warp], c, r);
+#pragma unroll
+                for (int q = 0; q < RQ; q++) rk[j + q] = r[q];
             }
             __syncthreads();
             {
