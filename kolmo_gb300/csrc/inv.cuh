@@ -10,7 +10,7 @@ struct InvBlock {
     u32 off;         // first byte of the block's BWT string (and of its decoded text)
     u32 n;           // block length
     u32 p0;          // primary index (row of the sentinel in the L column), 1..n
-    u32 chunk_base;  // first 64 KiB chunk of the block (psi build)
+    u32 chunk_base;  // first chunk of the block (psi build)
     u32 nchunk;
     u32 chain_base;  // first chain record of the block
     u32 nreg;        // regular marks: chain m in 1..nreg starts at row (m * hmul) & hmask when that row is <= n
@@ -53,11 +53,12 @@ class InvEngine {
     void layout(u64 ncap, u32 bcap, u64 tcap, u64 ccap, Add add);
     int build_graph(cudaStream_t s);
     int enqueue(cudaStream_t s, long long *launches);
+    u32 nmax() const;
     void free_all();
     u64 Ncap = 0, Tcap = 0, Ccap = 0;
     u32 Bcap = 0;
     u64 N = 0, nchunk_all = 0, nchains = 0;
-    u32 B = 0, maxchains = 0, njump = 0, nchunks = 0, nwalk = 0;
+    u32 B = 0, chunkt = 0, nchunks = 0, nwalk = 0;
     int walk_grid = 0;   // resident CTAs of the persistent walk kernel
     bool small = false;  // a small batch: denser marks and the persistent walk
     std::vector<u32> h_off;
@@ -66,7 +67,8 @@ class InvEngine {
     bool ext = false;
     u8 *d_U = nullptr, *d_out = nullptr, *own_U = nullptr, *own_out = nullptr;
     u32 *d_psi = nullptr, *d_csum = nullptr, *d_C = nullptr, *d_cblk = nullptr;
-    u32 *d_len = nullptr, *d_succ = nullptr, *d_nx[2] = {nullptr, nullptr}, *d_dist[2] = {nullptr, nullptr};
+    u32 *d_len = nullptr;
+    u64 *d_pair = nullptr;
     u32 *d_dyn = nullptr, *d_status = nullptr, *d_chunks = nullptr;
     u8 *d_buf = nullptr;
     InvBlock *d_blk = nullptr;
@@ -80,12 +82,12 @@ class InvEngine {
     // captured when it comes back
     struct GraphKey {
         u64 N, Ncap, nchunk_all, nchains;
-        u32 B, njump, nchunks;
+        u32 B, chunkt, nchunks, nmax;
         const void *U, *out;
         bool small;
         bool operator==(const GraphKey &o) const {
             return N == o.N && Ncap == o.Ncap && nchunk_all == o.nchunk_all && nchains == o.nchains && B == o.B &&
-                   njump == o.njump && nchunks == o.nchunks && U == o.U && out == o.out && small == o.small;
+                   chunkt == o.chunkt && nchunks == o.nchunks && nmax == o.nmax && U == o.U && out == o.out && small == o.small;
         }
     };
     GraphKey graph_key{}, seen_key{};
