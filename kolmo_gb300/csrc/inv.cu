@@ -34,17 +34,16 @@ namespace kgb {
 constexpr int ITPB = 256;
 constexpr u32 ITILE = 4096;
 constexpr u32 MARK = 64;
-// Small batches (at most SMALL_BATCH bytes, the drop-in call on a block of a few MiB) mark one row in MARK_SMALL and
-// walk on the persistent grid (k_inv_walk_flat): they have too few chains to fill the GPU otherwise. Larger batches
-// fill it with MARK and one CTA per work item (k_inv_walk), which is faster there (on a 64 MiB block: 3.38 ms for
-// the whole inverse against 3.66 with the persistent walk, 3.99 with one mark in 32 and 4.93 with one in 16; on a
-// 1 MiB block: 0.78 ms against 0.60, 0.50 and 0.46).
-constexpr u32 MARK_SMALL = 16;
-constexpr u64 SMALL_BATCH = 4u << 20;
+// Small batches (the drop-in call on a block of a few MiB) mark more rows: they have too few chains to fill the GPU
+// otherwise, and their walk is as long as the longest chain, about MARK ln(chains) rows. Whole inverse, one row in 64
+// / 16 / 8 / 4: 20 KB - / 79 / 69 / 63 us, 1 MiB - / 115 / 103 / 115 us; at 30 MB one in 32 takes 0.10 ms off the walk and
+// adds as much to the ranking and the copies.
+static u32 mark_of(u64 total) { return total <= 128u << 10 ? 4 : total <= 1536u << 10 ? 8 : total <= 4u << 20 ? 16 : MARK; }
 constexpr u32 CAPC = 256;
 constexpr u32 ENDC = 0xFFFFFFFFu;
-constexpr u32 CHUNK = 1024;  // start chains per walk work item
-constexpr int KSLOT = 4;     // chains walked at once by one thread
+// The byte of a row (its place in C) by a table over the rows' leading bits: entry i holds the byte values of the first
+// and last row of its range, and a search between the two (mostly none) ends the look-up.
+constexpr u32 FT_LOG = 10, FT = 1u << FT_LOG;
 // Tiles per chunk of the psi build: 16 on large batches, halved while the batch has at most CHUNKS_MIN chunks, so that
 // small ones fill the GPU (a 1 MiB block: 256 chunks of one tile instead of 16 of 16).
 constexpr u32 CHUNKT = 16, CHUNKS_MIN = 1024;
@@ -57,6 +56,7 @@ struct InvArgs {
     u32 *csum;
     const u32 *cblk;
     u32 *C;
+    u16 *ft;  // per block: FT entries, lowest byte value | highest << 8
     const InvBlock *blk;
     u32 B;
     u64 nchunk_all;
@@ -67,8 +67,6 @@ struct InvArgs {
     // and the length from its start to there. Read and written whole: both words always belong together.
     u64 *pair;
     u8 *buf;
-    const u32 *chunks;
-    u32 nchunks;
     u32 nwalk;  // chains in the walk's sequence over all blocks (sum of nreg + 1)
     u64 cap_n;  // bytes of the text buffers (checked build)
     u32 nmax;   // length of the longest block
@@ -86,6 +84,20 @@ __device__ __forceinline__ u32 chain_start(u32 id, const InvBlock &B) {
     if (id == 0) return B.p0;
     const u32 q = (id * B.hmul) & B.hmask;
     return q > B.n || q == B.p0 ? 0u : q;
+}
+
+// Rows of a block are 0..n; an entry of its byte table spans 2^ft_shift of them.
+__device__ __forceinline__ u32 ft_shift(u32 n) {
+    const u32 bits = 32 - __clz(n);
+    return bits > FT_LOG ? bits - FT_LOG : 0u;
+}
+// The largest c in [lo, hi] with C[c] <= row (C[lo] <= row).
+__device__ __forceinline__ u32 f_search(const u32 *Cs, u32 row, u32 lo, u32 hi) {
+    while (lo < hi) {
+        const u32 mid = (lo + hi + 1) >> 1;
+        if (Cs[mid] <= row) lo = mid; else hi = mid - 1;
+    }
+    return lo;
 }
 
 // Per-chunk byte histograms (a chunk is chunkt consecutive tiles of one block).
@@ -121,7 +133,7 @@ __global__ void __launch_bounds__(ITPB) k_inv_chunkhist(InvArgs a) {
 __global__ void __launch_bounds__(STPB) k_inv_chunkscan(InvArgs a) {
     __shared__ u32 ws[STPB / 32 + 1];
     __shared__ u32 part[4][256];
-    __shared__ u32 first[256];
+    __shared__ u32 first[257];
     const u32 c = threadIdx.x & 255, g = threadIdx.x >> 8;
     for (u32 b = blockIdx.x; b < a.B; b += gridDim.x) {
         const InvBlock B = a.blk[b];
@@ -146,9 +158,17 @@ __global__ void __launch_bounds__(STPB) k_inv_chunkscan(InvArgs a) {
         if (g == 0) {
             first[c] = cc;
             a.C[(u64)b * 257 + c] = cc;
-            if (c == 255) a.C[(u64)b * 257 + 256] = 1 + all;
+            if (c == 255) a.C[(u64)b * 257 + 256] = first[256] = 1 + all;
         }
         __syncthreads();
+        {
+            const u32 sh = ft_shift(B.n);
+            static_assert(FT == STPB, "one entry per thread");
+            const u64 r0 = (u64)threadIdx.x << sh, r1 = ((u64)(threadIdx.x + 1) << sh) - 1;
+            const u32 lo = f_search(first, (u32)max(r0, (u64)1), 0, 255);
+            const u32 hi = f_search(first, (u32)min(r1, (u64)B.n), 0, 255);
+            a.ft[(u64)b * FT + threadIdx.x] = (u16)(lo | max(lo, hi) << 8);
+        }
         u32 run = first[c];
         for (u32 w = 0; w < g; w++) run += part[w][c];
         q = q0;
@@ -230,100 +250,18 @@ __global__ void __launch_bounds__(ITPB, 3) k_inv_scatter(InvArgs a) {
     }
 }
 
-__device__ __forceinline__ u32 f_of(const u32 *Cs, u32 row) {  // largest c with C[c] <= row
-    u32 lo = 0;
-#pragma unroll
-    for (u32 step = 128; step; step >>= 1)
-        if (Cs[lo + step] <= row) lo += step;
-    return lo;
+constexpr int WALK_CTAS = 6;  // resident CTAs per SM of the walk
+// A random 4-byte load that leaves L1 to the byte tables.
+__device__ __forceinline__ u32 load_psi(const u32 *p) {
+    u32 v;
+    asm volatile("ld.global.nc.L1::no_allocate.u32 %0, [%1];" : "=r"(v) : "l"(p));
+    return v;
 }
 
 // A finished chain record: its bytes and its successor.
 __device__ __forceinline__ void close_chain(const InvArgs &a, u64 g, u32 len, u32 succ) {
     a.len[g] = len;
     a.pair[g] = (u64)succ << 32 | len;
-}
-
-// Walk every chain of a work item (block, [c0, c1) start chains). Chain 0 starts at p0; chain m >= 1 at its mark
-// (none when that row is past n or is p0). Chains that reach CAPC bytes continue under a new id taken from the block's counter.
-__global__ void __launch_bounds__(ITPB) k_inv_walk(InvArgs a) {
-    __shared__ u32 Cs[257];
-    for (u32 w = blockIdx.x; w < a.nchunks; w += gridDim.x) {
-        const u32 b = a.chunks[3 * w], c0 = a.chunks[3 * w + 1], c1 = a.chunks[3 * w + 2];
-        const InvBlock B = a.blk[b];
-        __syncthreads();
-        for (u32 i = threadIdx.x; i < 257; i += ITPB) Cs[i] = a.C[(u64)b * 257 + i];
-        __syncthreads();
-        const u32 *psi = a.psi + (u64)B.off + b;
-        u32 next = c0 + threadIdx.x;
-        u32 row[KSLOT], steps[KSLOT], acc[KSLOT], cid[KSLOT];
-        bool act[KSLOT];
-#pragma unroll
-        for (int k = 0; k < KSLOT; k++) {
-            act[k] = false;
-            while (next < c1) {
-                const u32 id = next;
-                next += ITPB;
-                const u32 start = chain_start(id, B);
-                if (start == 0) continue;  // no such row, or chain 0 covers the mark at p0
-                row[k] = start; steps[k] = 0; acc[k] = 0; cid[k] = id; act[k] = true;
-                break;
-            }
-        }
-        for (;;) {
-            bool any = false;
-            u32 v[KSLOT];
-#pragma unroll
-            for (int k = 0; k < KSLOT; k++)
-                if (act[k]) { v[k] = __ldg(psi + row[k]); any = true; }
-            if (!any) break;
-#pragma unroll
-            for (int k = 0; k < KSLOT; k++) {
-                if (!act[k]) continue;
-                const u64 g = (u64)B.chain_base + cid[k];
-                const u32 c = f_of(Cs, row[k]);
-                acc[k] |= c << (8 * (steps[k] & 3));
-                if ((steps[k] & 3) == 3) {
-                    reinterpret_cast<u32 *>(a.buf + g * CAPC)[steps[k] >> 2] = acc[k];
-                    acc[k] = 0;
-                }
-                steps[k]++;
-                u32 nxt = v[k] & 0x7FFFFFFFu;
-                if (nxt > B.n) {  // psi entries are rows 0..n: anything else is an internal error
-                    a.status[b] = 3;
-                    nxt = 0;
-                }
-                const bool stop = (v[k] >> 31) || nxt == 0;
-                if (stop || steps[k] == CAPC) {
-                    if (steps[k] & 3) reinterpret_cast<u32 *>(a.buf + g * CAPC)[steps[k] >> 2] = acc[k];
-                    if (stop) {
-                        close_chain(a, g, steps[k], nxt == 0 ? ENDC : B.chain_base + (nxt == B.p0 ? 0u : mark_id(nxt, B)));
-                        act[k] = false;
-                        while (next < c1) {
-                            const u32 id = next;
-                            next += ITPB;
-                            const u32 start = chain_start(id, B);
-                            if (start == 0) continue;
-                            row[k] = start; steps[k] = 0; acc[k] = 0; cid[k] = id; act[k] = true;
-                            break;
-                        }
-                    } else {
-                        const u32 nid = B.nreg + 1 + atomicAdd(&a.dyn[b], 1u);
-                        if (nid >= B.chain_cap) {  // cannot happen for any input: each record covers CAPC rows
-                            a.status[b] = 2;
-                            close_chain(a, g, steps[k], ENDC);
-                            act[k] = false;
-                        } else {
-                            close_chain(a, g, steps[k], B.chain_base + nid);
-                            cid[k] = nid; row[k] = nxt; steps[k] = 0; acc[k] = 0;
-                        }
-                    }
-                } else {
-                    row[k] = nxt;
-                }
-            }
-        }
-    }
 }
 
 // The block whose walk range holds chain q of the sequence over all blocks (blocks in order of qbase).
@@ -336,86 +274,90 @@ __device__ __forceinline__ u32 walk_block(const InvArgs &a, u32 q) {
     return lo;
 }
 
-// The walk as one sequence of chains over all blocks, on a persistent grid: thread t walks chains t, t + T,
-// t + 2T, ... (T threads in all), KSLOT at a time, and a slot takes the thread's next chain as soon as its chain
-// ends. Small batches use it: the work-item kernel above runs one CTA per 1024 chains, a few CTAs for a block of
-// a few MiB, while this one spreads the chains over every SM. Each step is the same as there.
-__global__ void __launch_bounds__(ITPB) k_inv_walk_flat(InvArgs a) {
-    __shared__ u32 Cs0[257];
-    const bool one = a.B == 1;  // a single block keeps its C array in shared memory
-    if (one) {
+// Walk every chain: chain 0 of a block starts at p0, chain m >= 1 at its mark (none when that row is past n or is p0).
+// Chains that reach CAPC bytes continue under a new id taken from the block's counter. ONE: the batch is one block,
+// whose byte tables fit shared memory (a batch of several reads them through L1, which the psi loads leave alone).
+//
+// Bound by the latency of dependent psi loads and by the lanes that wait for others. One chain per thread on a grid
+// that fills the GPU; CTA c takes runs c, c + G, c + 2G, ... of ITPB chains of the sequence, its threads the next of
+// them as they finish, so that the GPU works on one stretch of the sequence at a time and a batch's psi tables come
+// into L2 one after another. The load of the next row is issued before the current row's byte is looked up; bytes
+// leave in 16-byte words. On a 64 MiB block 1.52 ms (44 G rows/s; dependent random 4-byte loads over its 256 MiB table
+// reach 79 G/s), on 30 MB 0.69, on 1 MiB 0.05. Work items of 1024 chains, four to a thread, with 4-byte words took 2.16,
+// 1.10 and 0.09; with 4-byte words this walk takes 2.1 on 64 MiB: their partial sectors cost a quarter of it.
+template <bool ONE>
+__global__ void __launch_bounds__(ITPB, WALK_CTAS) k_inv_walk(InvArgs a) {
+    __shared__ u32 Cs0[ONE ? 257 : 1];
+    __shared__ u16 ft0[ONE ? FT : 1];
+    __shared__ u32 qnext;
+    if (threadIdx.x == 0) qnext = 0;
+    if (ONE) {
         for (u32 i = threadIdx.x; i < 257; i += ITPB) Cs0[i] = a.C[i];
-        __syncthreads();
+        for (u32 i = threadIdx.x; i < FT; i += ITPB) ft0[i] = a.ft[i];
     }
-    const u32 T = gridDim.x * ITPB;
-    u32 q = blockIdx.x * ITPB + threadIdx.x;
-    // per slot: current row, bytes so far, the word being filled, chain record, block, psi offset, block length
-    u32 row[KSLOT], steps[KSLOT], acc[KSLOT], grec[KSLOT], bk[KSLOT], pb[KSLOT], bn[KSLOT];
-    bool act[KSLOT];
-    // the thread's next chain into slot k (none left: the slot stays idle)
-#define KGB_TAKE(k)                                                                                              \
-    do {                                                                                                         \
-        act[k] = false;                                                                                          \
-        while (q < a.nwalk) {                                                                                    \
-            const u32 b_ = one ? 0u : walk_block(a, q);                                                          \
-            const InvBlock B_ = a.blk[b_];                                                                       \
-            const u32 id_ = q - B_.qbase;                                                                        \
-            q += T;                                                                                              \
-            const u32 st_ = chain_start(id_, B_);                                                                \
-            if (st_ == 0) continue; /* no such row, or chain 0 covers the mark at p0 */                        \
-            row[k] = st_; steps[k] = 0; acc[k] = 0; grec[k] = B_.chain_base + id_; bk[k] = b_;                 \
-            pb[k] = B_.off + b_; bn[k] = B_.n; act[k] = true;                                                   \
-            break;                                                                                               \
-        }                                                                                                        \
-    } while (0)
-#pragma unroll
-    for (int k = 0; k < KSLOT; k++) KGB_TAKE(k);
-    for (;;) {
-        bool any = false;
-        u32 v[KSLOT];
-#pragma unroll
-        for (int k = 0; k < KSLOT; k++)
-            if (act[k]) { v[k] = __ldg(a.psi + pb[k] + row[k]); any = true; }
-        if (!any) break;
-#pragma unroll
-        for (int k = 0; k < KSLOT; k++) {
-            if (!act[k]) continue;
-            const u32 *Cs = one ? Cs0 : a.C + (u64)bk[k] * 257;
-            acc[k] |= f_of(Cs, row[k]) << (8 * (steps[k] & 3));
-            steps[k]++;
-            u32 nxt = v[k] & 0x7FFFFFFFu;
-            if (nxt > bn[k]) {  // psi entries are rows 0..n: anything else is an internal error
-                a.status[bk[k]] = 3;
-                nxt = 0;
-            }
-            const bool stop = (v[k] >> 31) || nxt == 0;
-            if ((steps[k] & 3) == 0 || stop || steps[k] == CAPC) {
-                const u64 g = grec[k];
-                reinterpret_cast<u32 *>(a.buf + g * CAPC)[(steps[k] - 1) >> 2] = acc[k];
-                acc[k] = 0;
-                if (stop || steps[k] == CAPC) {
-                    const InvBlock B = a.blk[bk[k]];
-                    if (stop) {
-                        close_chain(a, g, steps[k], nxt == 0 ? ENDC : B.chain_base + (nxt == B.p0 ? 0u : mark_id(nxt, B)));
-                        KGB_TAKE(k);
-                    } else {
-                        const u32 nid = B.nreg + 1 + atomicAdd(&a.dyn[bk[k]], 1u);
-                        if (nid >= B.chain_cap) {  // cannot happen for any input: each record covers CAPC rows
-                            a.status[bk[k]] = 2;
-                            close_chain(a, g, steps[k], ENDC);
-                            act[k] = false;
-                        } else {
-                            close_chain(a, g, steps[k], B.chain_base + nid);
-                            grec[k] = B.chain_base + nid; row[k] = nxt; steps[k] = 0;
-                        }
-                    }
-                    continue;
+    __syncthreads();
+    u32 b = 0, sh = 0, bn = 0, row = 0, v = 0, steps = 0, rec = 0;
+    const u32 *psi = nullptr;
+    u64 a0 = 0, a1 = 0;  // the last 16 bytes, the latest on top
+    // the thread's next chain; false: none is left
+    auto take = [&]() -> bool {
+        for (;;) {
+            const u32 i = atomicAdd(&qnext, 1u);
+            const u64 q64 = ((u64)(i / ITPB) * gridDim.x + blockIdx.x) * ITPB + i % ITPB;
+            if (q64 >= a.nwalk) return false;
+            const u32 q = (u32)q64;
+            if (!ONE) b = walk_block(a, q);
+            const InvBlock B = a.blk[b];
+            const u32 id = q - B.qbase, start = chain_start(id, B);
+            if (start == 0) continue;  // no such row, or chain 0 covers the mark at p0
+            psi = a.psi + (u64)B.off + b;
+            bn = B.n;
+            sh = ft_shift(B.n);
+            row = start; steps = 0; rec = B.chain_base + id;
+            v = load_psi(psi + row);
+            return true;
+        }
+    };
+    bool act = take();
+    while (act) {
+        const u32 r = row, s = steps++;
+        u32 nxt = v & 0x7FFFFFFFu;
+        if (nxt > bn) {  // psi entries are rows 0..n: anything else is an internal error
+            a.status[b] = 3;
+            nxt = 0;
+        }
+        const bool stop = (v >> 31) || nxt == 0;
+        row = nxt;
+        if (!stop) v = load_psi(psi + nxt);
+        const u16 *ft = ONE ? ft0 : a.ft + (u64)b * FT;
+        const u32 t = ft[r >> sh];
+        const u32 c = f_search(ONE ? Cs0 : a.C + (u64)b * 257, r, t & 255u, t >> 8);
+        a0 = a0 >> 8 | a1 << 56;
+        a1 = a1 >> 8 | (u64)c << 56;
+        if ((s & 15) == 15 || stop) {
+            const u32 k = 8 * (15 - (s & 15));  // bits of the word not filled
+            const u64 lo = k == 0 ? a0 : k < 64 ? a0 >> k | a1 << (64 - k) : a1 >> (k - 64), hi = k < 64 ? a1 >> k : 0ull;
+            reinterpret_cast<ulonglong2 *>(a.buf + (u64)rec * CAPC)[s >> 4] = make_ulonglong2(lo, hi);
+        }
+        if (stop || s + 1 == CAPC) {
+            const InvBlock B = a.blk[b];
+            if (stop) {
+                close_chain(a, rec, s + 1, nxt == 0 ? ENDC : B.chain_base + (nxt == B.p0 ? 0u : mark_id(nxt, B)));
+                act = take();
+            } else {
+                const u32 nid = B.nreg + 1 + atomicAdd(&a.dyn[b], 1u);
+                if (nid >= B.chain_cap) {  // cannot happen for any input: each record covers CAPC rows
+                    a.status[b] = 2;
+                    close_chain(a, rec, s + 1, ENDC);
+                    act = take();
+                } else {
+                    close_chain(a, rec, s + 1, B.chain_base + nid);
+                    rec = B.chain_base + nid;
+                    steps = 0;
                 }
             }
-            row[k] = nxt;
         }
     }
-#undef KGB_TAKE
 }
 
 // Chain ranking by pointer jumping in place, in one launch: every record's pair (where its list of chains has been
@@ -507,13 +449,13 @@ void InvEngine::layout(u64 ncap, u32 bcap, u64 tcap, u64 ccap, Add add) {
     add((void **)&d_csum, tcap * 256 * 4);
     add((void **)&d_cblk, tcap * 4);
     add((void **)&d_C, (size_t)bcap * 257 * 4);
+    add((void **)&d_ft, (size_t)bcap * FT * 2);
     add((void **)&d_blk, (size_t)bcap * sizeof(InvBlock));
     add((void **)&d_len, ccap * 4);
     add((void **)&d_pair, ccap * 8);
     add((void **)&d_buf, ccap * CAPC);
     add((void **)&d_dyn, (size_t)bcap * 4);
     add((void **)&d_status, (size_t)bcap * 4);
-    add((void **)&d_chunks, (ccap / CHUNK + bcap + 8) * 12);
 }
 
 int InvEngine::grow(u64 ncap, u32 bcap, u64 tcap, u64 ccap) {
@@ -556,21 +498,19 @@ static void mark_params(InvBlock &B) {
     B.hinv = inv;
 }
 
-// A batch of at most SMALL_BATCH bytes (the persistent walk and denser marks).
-static bool small_batch(const u32 *n, int count) {
+static u32 mark_of(const u32 *n, int count) {
     u64 t = 0;
     for (int b = 0; b < count; b++) t += n[b];
-    return t <= SMALL_BATCH;
+    return mark_of(t);
 }
 
 static int plan_layout(const u32 *off, const u32 *n, const u32 *p0, int count, std::vector<InvBlock> &blk,
-                       std::vector<u32> &cblk, std::vector<u32> &chunks, u64 &nchunk_all, u64 &nchains, u32 &chunkt,
+                       std::vector<u32> &cblk, u64 &nchunk_all, u64 &nchains, u32 &chunkt,
                        u32 &nwalk) {
     blk.resize(count);
     nwalk = 0;
-    const u32 mark = small_batch(n, count) ? MARK_SMALL : MARK;
+    const u32 mark = mark_of(n, count);
     cblk.clear();
-    chunks.clear();
     nchunk_all = 0; nchains = 0;
     auto chunks_of = [&](u32 t) {
         u64 c = 0;
@@ -591,9 +531,6 @@ static int plan_layout(const u32 *off, const u32 *n, const u32 *p0, int count, s
         B.qbase = nwalk;
         nwalk += B.nreg + 1;
         for (u32 t = 0; t < B.nchunk; t++) cblk.push_back((u32)b);
-        for (u32 c = 0; c < B.nreg + 1; c += CHUNK) {
-            chunks.push_back((u32)b); chunks.push_back(c); chunks.push_back(std::min(B.nreg + 1, c + CHUNK));
-        }
         nchunk_all += B.nchunk;
         nchains += B.chain_cap;
         blk[b] = B;
@@ -607,10 +544,10 @@ u64 InvEngine::estimate_bytes(const u32 *n, int count) {
     u64 o = 0;
     for (int b = 0; b < count; b++) { off[b] = (u32)o; o += ((u64)n[b] + 15) / 16 * 16; }
     std::vector<InvBlock> blk;
-    std::vector<u32> cblk, chunks;
+    std::vector<u32> cblk;
     u64 nch = 0, nchains_ = 0;
     u32 ct = 0, nw = 0;
-    if (plan_layout(off.data(), n, p0.data(), count, blk, cblk, chunks, nch, nchains_, ct, nw)) return ~0ull;
+    if (plan_layout(off.data(), n, p0.data(), count, blk, cblk, nch, nchains_, ct, nw)) return ~0ull;
     u64 total = 0;
     layout(std::max<u64>(o, Ncap), std::max<u32>((u32)count, Bcap), std::max<u64>(nch, Tcap),
            std::max<u64>(nchains_, Ccap),
@@ -628,8 +565,7 @@ int InvEngine::plan(const u32 *n, const u32 *p0, int count) {
         if (off > 0xFFFF0000ull) return -1;
     }
     std::vector<u32> cblk;
-    if (plan_layout(h_off.data(), n, p0, count, h_blk, cblk, h_chunks, nchunk_all, nchains, chunkt, nwalk)) return -1;
-    small = small_batch(n, count);
+    if (plan_layout(h_off.data(), n, p0, count, h_blk, cblk, nchunk_all, nchains, chunkt, nwalk)) return -1;
     N = off; B = (u32)count;
     int rc = grow(N, B, nchunk_all, nchains);
     if (rc) return rc;
@@ -643,8 +579,7 @@ int InvEngine::plan_external(const u32 *off, const u32 *n, const u32 *p0, int co
     if (count <= 0) return -1;
     h_off.assign(off, off + count);
     std::vector<u32> cblk;
-    if (plan_layout(off, n, p0, count, h_blk, cblk, h_chunks, nchunk_all, nchains, chunkt, nwalk)) return -1;
-    small = small_batch(n, count);
+    if (plan_layout(off, n, p0, count, h_blk, cblk, nchunk_all, nchains, chunkt, nwalk)) return -1;
     u64 end = 0;
     for (int b = 0; b < count; b++) end = std::max<u64>(end, (u64)off[b] + n[b]);
     N = end; B = (u32)count;
@@ -665,10 +600,9 @@ u32 InvEngine::nmax() const {
 int InvEngine::enqueue(cudaStream_t s, long long *launches) {
     InvArgs a;
     memset(&a, 0, sizeof(a));
-    a.U = d_U; a.out = d_out; a.psi = d_psi; a.csum = d_csum; a.cblk = d_cblk; a.C = d_C; a.blk = d_blk; a.B = B;
+    a.U = d_U; a.out = d_out; a.psi = d_psi; a.csum = d_csum; a.cblk = d_cblk; a.C = d_C; a.ft = d_ft; a.blk = d_blk; a.B = B;
     a.nchunk_all = nchunk_all; a.chunkt = chunkt; a.nchains = nchains; a.len = d_len; a.pair = d_pair; a.dyn = d_dyn;
-    a.status = d_status; a.buf = d_buf;
-    a.chunks = d_chunks; a.nchunks = nchunks; a.nwalk = nwalk; a.cap_n = Ncap;
+    a.status = d_status; a.buf = d_buf; a.nwalk = nwalk; a.cap_n = Ncap;
     a.nmax = nmax();
     const int g8 = (int)std::min<u64>((u64)sm_count * 8, (nchains + ITPB - 1) / ITPB);
     KGB_CHECK(cudaMemsetAsync(d_len, 0, nchains * 4, s));
@@ -687,13 +621,12 @@ int InvEngine::enqueue(cudaStream_t s, long long *launches) {
     KGB_CHECK(go(K_INV_TILEHIST, nbytes, [&] { k_inv_chunkhist<<<gch, ITPB, 0, s>>>(a); }));
     KGB_CHECK(go(K_INV_COLSCAN, (u32)nchunk_all, [&] { k_inv_chunkscan<<<(int)std::min<u32>(B, 4096u), STPB, 0, s>>>(a); }));
     KGB_CHECK(go(K_INV_SCATTER, nbytes, [&] { k_inv_scatter<<<gch, ITPB, 0, s>>>(a); }));
-    if (small) {
-        // the persistent grid: the CTAs the GPU holds at once, or fewer when there are fewer chains than threads
-        const int gw = (int)std::max<u64>(1, std::min<u64>((u64)walk_grid, ((u64)nwalk + ITPB - 1) / ITPB));
-        KGB_CHECK(go(K_INV_WALK, nbytes, [&] { k_inv_walk_flat<<<gw, ITPB, 0, s>>>(a); }));
-    } else {
-        KGB_CHECK(go(K_INV_WALK, nbytes, [&] { k_inv_walk<<<(int)std::min<u32>(nchunks, (u32)sm_count * 8), ITPB, 0, s>>>(a); }));
-    }
+    // the CTAs the GPU holds at once, or fewer when there are fewer chains than threads
+    const int gw = (int)std::max<u64>(1, std::min<u64>((u64)walk_grid, ((u64)nwalk + ITPB - 1) / ITPB));
+    KGB_CHECK(go(K_INV_WALK, nbytes, [&] {
+        if (B == 1) k_inv_walk<true><<<gw, ITPB, 0, s>>>(a);
+        else k_inv_walk<false><<<gw, ITPB, 0, s>>>(a);
+    }));
     KGB_CHECK(go(K_INV_JUMP, (u32)nchains, [&] { k_inv_rank<<<g8, ITPB, 0, s>>>(a); }));
     KGB_CHECK(go(K_INV_EMIT, nbytes, [&] { k_inv_emit<<<sm_count * 8, ITPB, 0, s>>>(a); }));
     return 0;
@@ -705,20 +638,16 @@ int InvEngine::run(cudaStream_t s, bool use_graph) {
         int dev;
         KGB_CHECK(cudaGetDevice(&dev));
         KGB_CHECK(cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev));
-        int per_sm = 0;
-        KGB_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_inv_walk_flat, ITPB, 0));
-        walk_grid = std::max(per_sm, 1) * sm_count;
+        walk_grid = WALK_CTAS * sm_count;
     }
-    nchunks = (u32)(h_chunks.size() / 3);
     stats.jumps = 1;
     KGB_CHECK(cudaMemcpyAsync(d_blk, h_blk.data(), h_blk.size() * sizeof(InvBlock), cudaMemcpyHostToDevice, s));
-    KGB_CHECK(cudaMemcpyAsync(d_chunks, h_chunks.data(), h_chunks.size() * 4, cudaMemcpyHostToDevice, s));
     KGB_CHECK(cudaStreamSynchronize(s));  // host vectors are pageable: finish before they can change
     prof.reset();
     prof_run = !use_graph && prof.on;
     if (!use_graph) return enqueue(s, &stats.launches);
     prof_run = false;
-    const GraphKey key{N, Ncap, (u64)nchunk_all, (u64)nchains, (u32)B, chunkt, nchunks, nmax(), d_U, d_out, small};
+    const GraphKey key{N, Ncap, (u64)nchunk_all, (u64)nchains, (u32)B, chunkt, nwalk, nmax(), d_U, d_out};
     if (!gexec || !(key == graph_key)) {
         if (!(seen_valid && key == seen_key)) {  // first sight of this shape: plain launches, no capture
             seen_key = key;
@@ -765,19 +694,18 @@ constexpr u32 NOALLOC_MAX_N = 1u << 18;  // 256 KiB
 constexpr u32 NA_CHUNKS = NOALLOC_MAX_N / ITILE;  // chunks of one tile
 constexpr u32 NA_NREG = NOALLOC_MAX_N / MARK;
 constexpr u32 NA_CHAINS = NA_NREG + 1 + NOALLOC_MAX_N / CAPC + 4;
-constexpr u32 NA_WALK = (NA_NREG + 1 + CHUNK - 1) / CHUNK;
 
 struct NoAllocScratch {
     u32 psi[NOALLOC_MAX_N + 16];
     u32 csum[NA_CHUNKS * 256];
     u32 C[264];
+    u16 ft[FT];
     u32 cblk[NA_CHUNKS];
-    u32 chunks[3 * NA_WALK];
     InvBlock blk[1];
     u64 pair[NA_CHAINS];
     u32 len[NA_CHAINS];
     u32 dyn[4], status[4];
-    u8 buf[(size_t)NA_CHAINS * CAPC];
+    __align__(16) u8 buf[(size_t)NA_CHAINS * CAPC];
 };
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[sizeof(NoAllocScratch)];
@@ -805,21 +733,15 @@ static int unbwt_noalloc(const u8 *dU, u8 *dT, u32 n, u32 p0, cudaStream_t s) {
     int rc = 0;
     NoAllocScratch *S = noalloc_scratch(&rc);
     if (!S) return rc;
-    // host-side tables on the stack: one block, its chunk map and its walk work items
+    // host-side tables on the stack: one block and its chunk map
     InvBlock B;
     B.off = 0; B.n = n; B.p0 = p0;
     B.chunk_base = 0; B.nchunk = (n + ITILE - 1) / ITILE;
     B.nreg = n / MARK; B.chain_base = 0; B.chain_cap = B.nreg + 1 + n / CAPC + 4; B.qbase = 0;
     mark_params(B);
     u32 cblk[NA_CHUNKS] = {0};
-    u32 chunks[3 * NA_WALK];
-    u32 nwalk = 0;
-    for (u32 c = 0; c < B.nreg + 1; c += CHUNK, nwalk++) {
-        chunks[3 * nwalk] = 0; chunks[3 * nwalk + 1] = c; chunks[3 * nwalk + 2] = std::min(B.nreg + 1, c + CHUNK);
-    }
     KGB_CHECK(cudaMemcpyAsync(S->blk, &B, sizeof(B), cudaMemcpyHostToDevice, s));
     KGB_CHECK(cudaMemcpyAsync(S->cblk, cblk, sizeof(u32) * B.nchunk, cudaMemcpyHostToDevice, s));
-    KGB_CHECK(cudaMemcpyAsync(S->chunks, chunks, sizeof(u32) * 3 * nwalk, cudaMemcpyHostToDevice, s));
     // the array keeps the previous call's contents: reset what must start at zero (or at "no successor")
     KGB_CHECK(cudaMemsetAsync(S->len, 0, sizeof(u32) * B.chain_cap, s));
     KGB_CHECK(cudaMemsetAsync(S->pair, 0xFF, sizeof(u64) * B.chain_cap, s));
@@ -827,13 +749,13 @@ static int unbwt_noalloc(const u8 *dU, u8 *dT, u32 n, u32 p0, cudaStream_t s) {
     KGB_CHECK(cudaMemsetAsync(S->status, 0, sizeof(S->status), s));
     InvArgs a;
     memset(&a, 0, sizeof(a));
-    a.U = dU; a.out = dT; a.psi = S->psi; a.csum = S->csum; a.cblk = S->cblk; a.C = S->C; a.blk = S->blk; a.B = 1;
+    a.U = dU; a.out = dT; a.psi = S->psi; a.csum = S->csum; a.cblk = S->cblk; a.C = S->C; a.ft = S->ft; a.blk = S->blk; a.B = 1;
     a.nchunk_all = B.nchunk; a.chunkt = 1; a.nchains = B.chain_cap; a.len = S->len; a.pair = S->pair; a.dyn = S->dyn;
-    a.status = S->status; a.buf = S->buf; a.chunks = S->chunks; a.nchunks = nwalk; a.cap_n = n; a.nmax = n;
+    a.status = S->status; a.buf = S->buf; a.nwalk = B.nreg + 1; a.cap_n = n; a.nmax = n;
     k_inv_chunkhist<<<B.nchunk, ITPB, 0, s>>>(a);
     k_inv_chunkscan<<<1, STPB, 0, s>>>(a);
     k_inv_scatter<<<B.nchunk, ITPB, 0, s>>>(a);
-    k_inv_walk<<<nwalk, ITPB, 0, s>>>(a);
+    k_inv_walk<true><<<(B.nreg + ITPB) / ITPB, ITPB, 0, s>>>(a);
     const int g = (int)((B.chain_cap + ITPB - 1) / ITPB);
     k_inv_rank<<<g, ITPB, 0, s>>>(a);
     k_inv_emit<<<8 * g, ITPB, 0, s>>>(a);

@@ -58,18 +58,17 @@ class InvEngine {
     u64 Ncap = 0, Tcap = 0, Ccap = 0;
     u32 Bcap = 0;
     u64 N = 0, nchunk_all = 0, nchains = 0;
-    u32 B = 0, chunkt = 0, nchunks = 0, nwalk = 0;
-    int walk_grid = 0;   // resident CTAs of the persistent walk kernel
-    bool small = false;  // a small batch: denser marks and the persistent walk
+    u32 B = 0, chunkt = 0, nwalk = 0;
+    int walk_grid = 0;   // resident CTAs of the walk kernel
     std::vector<u32> h_off;
     std::vector<InvBlock> h_blk;
-    std::vector<u32> h_chunks;  // (block, first chain, end chain) triples for the walk
     bool ext = false;
     u8 *d_U = nullptr, *d_out = nullptr, *own_U = nullptr, *own_out = nullptr;
     u32 *d_psi = nullptr, *d_csum = nullptr, *d_C = nullptr, *d_cblk = nullptr;
     u32 *d_len = nullptr;
     u64 *d_pair = nullptr;
-    u32 *d_dyn = nullptr, *d_status = nullptr, *d_chunks = nullptr;
+    u32 *d_dyn = nullptr, *d_status = nullptr;
+    u16 *d_ft = nullptr;
     u8 *d_buf = nullptr;
     InvBlock *d_blk = nullptr;
     void *pool = nullptr;
@@ -82,12 +81,11 @@ class InvEngine {
     // captured when it comes back
     struct GraphKey {
         u64 N, Ncap, nchunk_all, nchains;
-        u32 B, chunkt, nchunks, nmax;
+        u32 B, chunkt, nwalk, nmax;
         const void *U, *out;
-        bool small;
         bool operator==(const GraphKey &o) const {
             return N == o.N && Ncap == o.Ncap && nchunk_all == o.nchunk_all && nchains == o.nchains && B == o.B &&
-                   chunkt == o.chunkt && nchunks == o.nchunks && nmax == o.nmax && U == o.U && out == o.out && small == o.small;
+                   chunkt == o.chunkt && nwalk == o.nwalk && nmax == o.nmax && U == o.U && out == o.out;
         }
     };
     GraphKey graph_key{}, seen_key{};

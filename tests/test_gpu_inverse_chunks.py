@@ -1,6 +1,7 @@
-"""The inverse's psi build, chain ranking and copy at the sizes where they change shape: chunk and tile edges (4096
-bytes, one tile per chunk on small batches), the switch from the persistent walk to work items (4 MiB), output blocks at
-every byte alignment, and strings with several cycles (not a BWT: reported, whatever the ranking meets on them)."""
+"""The inverse's psi build, chain walk, ranking and copy at the sizes where they change shape: chunk and tile edges
+(4096 bytes, one tile per chunk on small batches), the steps of the mark density (128 KiB, 1.5 MiB, 4 MiB of input),
+output blocks at every byte alignment, and strings with several cycles (not a BWT: reported, whatever the ranking meets
+on them)."""
 import numpy as np
 import pytest
 
@@ -19,7 +20,8 @@ def _text(n, seed):
     return t
 
 
-@pytest.mark.parametrize("n", [2, 3, 5, 255, 4095, 4096, 4097, 8191, 65535, 65537, (1 << 20) - 1, (1 << 20) + 1])
+@pytest.mark.parametrize("n", [2, 3, 5, 255, 4095, 4096, 4097, 8191, 65535, 65537, (128 << 10) - 1,
+                               (128 << 10) + 1, (1 << 20) - 1, (1 << 20) + 1, (1536 << 10) + 1])
 def test_round_trip_at_chunk_edges(n):
     T = _text(n, n)
     rc, U, I = O.bwt_aux(T, 1 << 30)
@@ -30,7 +32,7 @@ def test_round_trip_at_chunk_edges(n):
 
 
 @pytest.mark.parametrize("total", [(4 << 20) - 3, (4 << 20) + 5])
-def test_batch_around_the_walk_switch(total):
+def test_batch_around_a_mark_density_step(total):
     import torch
 
     sizes = [17, 4099, 70001, 300007, 3]
