@@ -250,13 +250,11 @@ __global__ void __launch_bounds__(ITPB, 3) k_inv_scatter(InvArgs a) {
     }
 }
 
-constexpr int WALK_CTAS = 6;  // resident CTAs per SM of the walk
-// A random 4-byte load that leaves L1 to the byte tables.
-__device__ __forceinline__ u32 load_psi(const u32 *p) {
-    u32 v;
-    asm volatile("ld.global.nc.L1::no_allocate.u32 %0, [%1];" : "=r"(v) : "l"(p));
-    return v;
-}
+// CTAs per SM of the walk. More chains in flight spread over more blocks of a batch, whose psi tables then push each
+// other out of L2 (mixed batch: 2.75 ms with 3, 4.16 with 6, 4.18 with 1; a 64 MiB block 1.36, 1.41 and 1.86).
+constexpr int WALK_CTAS = 3;
+constexpr int WSTEP = 8;  // rows between two looks at finished chains (one 8-byte word of text)
+static_assert(CAPC % (2 * WSTEP) == 0, "records fill with whole 16-byte words");
 
 // A finished chain record: its bytes and its successor.
 __device__ __forceinline__ void close_chain(const InvArgs &a, u64 g, u32 len, u32 succ) {
@@ -276,17 +274,18 @@ __device__ __forceinline__ u32 walk_block(const InvArgs &a, u32 q) {
 
 // Walk every chain: chain 0 of a block starts at p0, chain m >= 1 at its mark (none when that row is past n or is p0).
 // Chains that reach CAPC bytes continue under a new id taken from the block's counter. ONE: the batch is one block,
-// whose byte tables fit shared memory (a batch of several reads them through L1, which the psi loads leave alone).
+// whose byte tables fit shared memory (a batch of several reads them through L1).
 //
-// Bound by the latency of dependent psi loads and by the lanes that wait for others. One chain per thread on a grid
-// that fills the GPU; CTA c takes runs c, c + G, c + 2G, ... of ITPB chains of the sequence, its threads the next of
-// them as they finish, so that the GPU works on one stretch of the sequence at a time and a batch's psi tables come
-// into L2 one after another. The load of the next row is issued before the current row's byte is looked up; bytes
-// leave in 16-byte words. On a 64 MiB block 1.52 ms (44 G rows/s; dependent random 4-byte loads over its 256 MiB table
-// reach 79 G/s), on 30 MB 0.69, on 1 MiB 0.05. Work items of 1024 chains, four to a thread, with 4-byte words took 2.16,
-// 1.10 and 0.09; with 4-byte words this walk takes 2.1 on 64 MiB: their partial sectors cost a quarter of it.
+// Bound by dependent random psi loads: 77 G rows/s over the small blocks of a batch, 49 G on a 64 MiB block, whose
+// 256 MiB table is twice L2 (independent 4-byte loads reach 79 G/s there, 280 where the table fits). One chain per
+// thread; CTA c takes runs c, c + G, c + 2G, ... of ITPB chains of the sequence, its threads the next of them as they
+// finish, so that the GPU works on one stretch of the sequence at a time. Chains are closed, stored and replaced only
+// every WSTEP rows (an ended chain waits 4 rows of about 64), so that a warp runs that code once for all its lanes; the
+// load of the next row is issued before the current row's byte is looked up; bytes leave in 16-byte words (4-byte words
+// cost a quarter of the walk in partial sectors). The psi loads keep the default cache policy: L1::no_allocate marks
+// their lines for early eviction from L2 too and took 4.13 ms where this takes 2.75 (mixed batch).
 template <bool ONE>
-__global__ void __launch_bounds__(ITPB, WALK_CTAS) k_inv_walk(InvArgs a) {
+__global__ void __launch_bounds__(ITPB, 6) k_inv_walk(InvArgs a) {
     __shared__ u32 Cs0[ONE ? 257 : 1];
     __shared__ u16 ft0[ONE ? FT : 1];
     __shared__ u32 qnext;
@@ -298,7 +297,6 @@ __global__ void __launch_bounds__(ITPB, WALK_CTAS) k_inv_walk(InvArgs a) {
     __syncthreads();
     u32 b = 0, sh = 0, bn = 0, row = 0, v = 0, steps = 0, rec = 0;
     const u32 *psi = nullptr;
-    u64 a0 = 0, a1 = 0;  // the last 16 bytes, the latest on top
     // the thread's next chain; false: none is left
     auto take = [&]() -> bool {
         for (;;) {
@@ -314,44 +312,60 @@ __global__ void __launch_bounds__(ITPB, WALK_CTAS) k_inv_walk(InvArgs a) {
             bn = B.n;
             sh = ft_shift(B.n);
             row = start; steps = 0; rec = B.chain_base + id;
-            v = load_psi(psi + row);
+            v = __ldg(psi + row);
             return true;
         }
     };
     bool act = take();
-    while (act) {
-        const u32 r = row, s = steps++;
-        u32 nxt = v & 0x7FFFFFFFu;
-        if (nxt > bn) {  // psi entries are rows 0..n: anything else is an internal error
-            a.status[b] = 3;
-            nxt = 0;
+    u64 prev = 0, cur = 0;  // the chain's last two 8-byte words
+    // (the vote brings the warp's lanes together again: left to themselves they drift apart, nine to an instruction)
+    while (__any_sync(0xffffffffu, act)) {
+        // WSTEP rows; a lane whose chain ends waits for the others
+        bool live = act;
+        cur = 0;
+#pragma unroll
+        for (int j = 0; j < WSTEP; j++) {
+            const bool go = live;
+            const u32 r = row;
+            if (go) {
+                u32 nxt = v & 0x7FFFFFFFu;
+                if (nxt > bn) {  // psi entries are rows 0..n: anything else is an internal error
+                    a.status[b] = 3;
+                    nxt = 0;
+                }
+                live = !(v >> 31) && nxt != 0;
+                row = nxt;
+                if (live) v = __ldg(psi + nxt);
+                steps++;
+            }
+            u32 c = 0;
+            if (go) {
+                const u16 *ft = ONE ? ft0 : a.ft + (u64)b * FT;
+                const u32 t = ft[r >> sh];
+                c = f_search(ONE ? Cs0 : a.C + (u64)b * 257, r, t & 255u, t >> 8);
+            }
+            cur = cur >> 8 | (u64)c << 56;
+            __syncwarp();
         }
-        const bool stop = (v >> 31) || nxt == 0;
-        row = nxt;
-        if (!stop) v = load_psi(psi + nxt);
-        const u16 *ft = ONE ? ft0 : a.ft + (u64)b * FT;
-        const u32 t = ft[r >> sh];
-        const u32 c = f_search(ONE ? Cs0 : a.C + (u64)b * 257, r, t & 255u, t >> 8);
-        a0 = a0 >> 8 | a1 << 56;
-        a1 = a1 >> 8 | (u64)c << 56;
-        if ((s & 15) == 15 || stop) {
-            const u32 k = 8 * (15 - (s & 15));  // bits of the word not filled
-            const u64 lo = k == 0 ? a0 : k < 64 ? a0 >> k | a1 << (64 - k) : a1 >> (k - 64), hi = k < 64 ? a1 >> k : 0ull;
-            reinterpret_cast<ulonglong2 *>(a.buf + (u64)rec * CAPC)[s >> 4] = make_ulonglong2(lo, hi);
-        }
-        if (stop || s + 1 == CAPC) {
-            const InvBlock B = a.blk[b];
-            if (stop) {
-                close_chain(a, rec, s + 1, nxt == 0 ? ENDC : B.chain_base + (nxt == B.p0 ? 0u : mark_id(nxt, B)));
+        if (act) {
+            const u32 w = (steps - 1) / WSTEP;
+            if (w & 1 || !live)
+                reinterpret_cast<ulonglong2 *>(a.buf + (u64)rec * CAPC)[w >> 1] =
+                    w & 1 ? make_ulonglong2(prev, cur) : make_ulonglong2(cur, 0);
+            prev = cur;
+            if (!live) {
+                const InvBlock B = a.blk[b];
+                close_chain(a, rec, steps, row == 0 ? ENDC : B.chain_base + (row == B.p0 ? 0u : mark_id(row, B)));
                 act = take();
-            } else {
+            } else if (steps == CAPC) {
+                const InvBlock B = a.blk[b];
                 const u32 nid = B.nreg + 1 + atomicAdd(&a.dyn[b], 1u);
                 if (nid >= B.chain_cap) {  // cannot happen for any input: each record covers CAPC rows
                     a.status[b] = 2;
-                    close_chain(a, rec, s + 1, ENDC);
+                    close_chain(a, rec, steps, ENDC);
                     act = take();
                 } else {
-                    close_chain(a, rec, s + 1, B.chain_base + nid);
+                    close_chain(a, rec, steps, B.chain_base + nid);
                     rec = B.chain_base + nid;
                     steps = 0;
                 }
