@@ -436,19 +436,6 @@ __global__ void __launch_bounds__(TPB) k_lsd_hist0(FwdArgs a) {
     }
 }
 
-// When no key byte varies within any block, no pass runs: the sorted order is the text order (ids written here for
-// the segmentation). Otherwise returns at once.
-__global__ void __launch_bounds__(TPB) k_lsd_ident(FwdArgs a) {
-    const Ctl *c = a.ctl;
-    if (active_slots(c)) return;
-    const u32 nt = c->lsd_tiles;
-    for (u32 t = blockIdx.x; t < nt; t += gridDim.x) {
-        const LsdTile tl = lsd_tile(a, t);
-        const u32 id0 = a.blk[tl.b].off + (tl.base - a.blk[tl.b].soff);
-        for (u32 j = threadIdx.x; j < tl.cnt; j += TPB) __stcs(a.lval[0] + tl.base + j, id0 + j);
-    }
-}
-
 constexpr int RANK_Q = 4;  // elements a lane ranks at once
 struct LsdSmem {
     unsigned long long item[LSD_TILE];
@@ -646,8 +633,16 @@ __global__ void __launch_bounds__(TPB, 3) k_lsd_pass(FwdArgs a, int slot) {
     LsdSmem &S = *reinterpret_cast<LsdSmem *>(smem_raw);
     const Ctl *c = a.ctl;
     const u32 act = active_slots(c);
-    if (!((act >> slot) & 1)) return;
     const u32 ntiles = c->lsd_tiles;
+    if (!((act >> slot) & 1)) {
+        // no key byte varies within any block: the sorted order is the text order, written by the first slot's launch
+        if (act == 0 && slot == 16 - (int)a.lsd_bytes && blockIdx.x < ntiles) {
+            const LsdTile tl = lsd_tile(a, blockIdx.x);
+            const u32 id0 = a.blk[tl.b].off + (tl.base - a.blk[tl.b].soff);
+            for (u32 j = threadIdx.x; j < tl.cnt; j += TPB) __stcs(a.lval[0] + tl.base + j, id0 + j);
+        }
+        return;
+    }
     const u64 epoch = (u64)((c->seq << 5) | (u32)slot) << 32;
     const u32 tid = threadIdx.x;
     if (tid == 0) S.tile = atomicAdd(&a.ltile[slot], 1u);
