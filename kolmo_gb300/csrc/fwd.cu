@@ -51,7 +51,15 @@ constexpr u32 STABLE = 0x80000000u;
 // the top byte of the groups they split; those start again from h.)
 constexpr u32 DEPTH_SHIFT = 24, DEPTH_MAX = 127;
 
-enum : u8 { C_NONE = 0, C_KS = 1, C_KO = 2, C_LN = 3, C_ONE = 4 };
+// Rank labels of large groups. The rank of a suffix in a group need not be the group's first position: any position of
+// the group's range orders the groups alike, so a bucket that holds its parent's label keeps it, and its members' ranks
+// need no writing (the others take their middle, which the largest part of a later split is likely to hold). lab[s] is
+// the label of group s, with LAB_BOTH when the write buffer holds it for every member as well. On a periodic block each
+// round cuts a few members off every group: writing the whole block's ranks again was half of a round (128 MiB of
+// 4096-byte records: 5.8 ms of bucket scatters a round).
+constexpr u32 LAB_BOTH = 0x80000000u;
+
+enum : u8 { C_NONE = 0, C_KS = 1, C_KO = 2, C_LN = 3, C_ONE = 4, C_LK = 5 };  // C_LK: C_LN whose ranks stand
 
 struct FwdArgs {
     Ctl *ctl;
@@ -1578,6 +1586,10 @@ __global__ void __launch_bounds__(TPB) k_msd_scan(FwdArgs a) {
         }
         __syncthreads();
         const u32 head = g.head + excl, blk = seg_blk(g.bd);
+        // the bucket's rank label: its parent's when that lies in its range (after a prefix round: its first position)
+        const u32 plab = PREFIX ? 0u : in.lab[s];
+        const bool kept = !PREFIX && (plab & ~LAB_BOTH) - head < cc;
+        const u32 label = PREFIX ? head : kept ? plab & ~LAB_BOTH : head + cc / 2;
         u32 nb = 0, t0 = 0, sidx = 0;
         if (cls == C_ONE) {
             a.cursor[hrow + tid] = S.base_e[C_ONE] + x_one;  // slot in the resolved list
@@ -1591,7 +1603,13 @@ __global__ void __launch_bounds__(TPB) k_msd_scan(FwdArgs a) {
             Seg ng;
             ng.start = start; ng.len = cc; ng.head = head; ng.bd = bd;
             KGB_GUARD(sidx < (cls == C_KS ? a.cap_segk : a.cap_segl) && (u64)start + cc <= a.cap_n, &a.ctl->err, E_SEG)
-            o.seg[sidx] = ng;
+            {
+                o.seg[sidx] = ng;
+                // a bucket to be split further carries the group's label on; a finished one holds its own in the buffer
+                // this round writes, and in the other one too when it kept the group's
+                if (cls == C_KO) o.lab[sidx] = plab;
+                if (cls == C_LN) o.lab[sidx] = label | (kept ? LAB_BOTH : 0u);
+            }
             a.cursor[hrow + tid] = start;
             if (cls == C_KS) {
                 write_tmap_small(a, o.tmap, a.smax, start, cc, sidx);
@@ -1602,8 +1620,8 @@ __global__ void __launch_bounds__(TPB) k_msd_scan(FwdArgs a) {
                 nb = t1 >= t0 ? t1 - t0 + 1 : 0;
             }
         }
-        a.bhead[hrow + tid] = head;
-        a.dest[hrow + tid] = cls;
+        a.bhead[hrow + tid] = cls == C_LN ? label : head;
+        a.dest[hrow + tid] = cls == C_LN && kept && (plab & LAB_BOTH) ? C_LK : cls;
         __syncthreads();  // every thread has read orand64[s]
         if (PREFIX && tid == 0) { a.orand64[2 * s] = 0; a.orand64[2 * s + 1] = ~0ull; }
         if (!PREFIX && pass == 0 && tid == 0) {  // the scatter reads the digit from the descriptor
@@ -1699,9 +1717,9 @@ __global__ void __launch_bounds__(TPB) k_msd_scatter(FwdArgs a) {
             } else if (cls == C_KO) {
                 ko.eid[pos] = id;
                 if (!PREFIX) ko.ekey[pos] = keys[j];
-            } else if (cls == C_LN) {
+            } else if (cls == C_LN || cls == C_LK) {
                 ln.eid[pos] = id;
-                isa_nxt[id] = a.bhead[row];
+                if (cls == C_LN) isa_nxt[id] = a.bhead[row];
             } else {  // C_ONE
                 resolve(a, isa_nxt, id, a.bhead[row], seg_blk((sel ? m.g1 : m.g0).bd), res, pos);
             }
@@ -1813,7 +1831,7 @@ __global__ void k_init(FwdArgs a, const u32 *__restrict__ blk_list_start, const 
 static size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 
 FwdEngine::FwdEngine() {
-    for (auto &l : lists) l = ListView{nullptr, nullptr, nullptr, nullptr};
+    for (auto &l : lists) l = ListView{};
 }
 FwdEngine::~FwdEngine() { free_all(); }
 
@@ -1870,6 +1888,7 @@ void FwdEngine::layout(u64 ncap, u32 bcap, u32 icap, bool want_sa, Add add) {
             add((void **)&lists[l].seg, (l == L_KS ? nseg_small : small ? nseg_s : nseg_large) * sizeof(Seg));
             add((void **)&lists[l].tmap, (small ? ntm_small : ntm_large) * 4);
             if (small) add((void **)&lists[l].tbig, ntm_small * 4);
+            else add((void **)&lists[l].lab, nseg_large * 4);
         }
     }
     add((void **)&d_hist, nseg_large * 256 * 4);
@@ -1915,7 +1934,7 @@ int FwdEngine::grow(u64 ncap, u32 bcap, u32 icap, bool want_sa) {
     if (graph) { cudaGraphDestroy(graph); graph = nullptr; }
     if (pool) { cudaFree(pool); pool = nullptr; }
     own_SA = nullptr;
-    for (auto &l : lists) l = ListView{nullptr, nullptr, nullptr, nullptr};
+    for (auto &l : lists) l = ListView{};
     struct Item { void **p; size_t bytes; };
     std::vector<Item> items;
     layout(ncap, bcap, icap, want_sa,

@@ -39,6 +39,7 @@ struct ListView {
     u32 *eid;   // element: global suffix index
     u32 *ekey;  // element: current sort key (rank rounds), may be null
     Seg *seg;   // segment descriptors
+    u32 *lab;   // large and bucket-pass lists: each group's rank label (see LAB_BOTH in fwd.cu)
     u32 *tmap;  // tile map (see fwd.cu)
     u32 *tbig;  // small lists: per tile window, the round stamp of a group longer than WARP_GROUP starting there
 };

@@ -1013,6 +1013,7 @@ __global__ void __launch_bounds__(TPB) k_seg_emit1(FwdArgs a) {
                     g.start = le;
                     KGB_GUARD(lidx < a.cap_segl && (u64)le + len <= a.cap_n, &c->err, E_SEG) {
                         ll.seg[lidx] = g;
+                        ll.lab[lidx] = head | LAB_BOTH;  // (round 1's fixup copies every rank to the other buffer)
                         v.gbase[gf] = le;
                         v.gidx[gf] = lidx | GRP_LARGE;
                     }
