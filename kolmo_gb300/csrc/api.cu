@@ -39,6 +39,14 @@ int record_cuda_error(cudaError_t e, const char *what, const char *file, int lin
     return -2;
 }
 
+int refuse_capture(cudaStream_t s) {
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    KGB_CHECK(cudaStreamIsCapturing(s, &cs));
+    if (cs == cudaStreamCaptureStatusNone) return 0;
+    record_error("the stream is being captured; this call reads host memory and cannot be recorded");
+    return -2;
+}
+
 int Pinned::need(size_t bytes) {
     if (bytes <= cap) return 0;
     release();
@@ -120,6 +128,20 @@ static bool page_locked(const void *p) {
     return at.type == cudaMemoryTypeHost || at.type == cudaMemoryTypeManaged;
 }
 
+// Results of this many bytes go straight into the caller's buffer, smaller ones through pinned staging and a host copy:
+// copying 30 MB from staging takes 2.2 ms on one core (2.7 into pages not yet touched), 1 MiB 40 us, where the device
+// writes either in 0.17 ms and 15 us; below, the second wait for the stream costs more (about 10 us).
+constexpr size_t DIRECT_MIN = 512u << 10;
+enum : u8 { D_STAGED = 0, D_PAGEABLE = 1, D_LOCKED = 2 };
+
+// Maps the caller's buffer while the device works: the device's writes to a page that the process has not touched yet
+// take 100 times as long (26 ms for 30 MB of fresh pages). An atomic OR with nothing keeps every byte and is a write from
+// the first access on (a read first would map the shared zero page and split huge pages: 8 ms for 30 MB).
+static void touch_pages(u8 *p, size_t n) {
+    for (size_t i = 0; i < n; i += 4096) __atomic_fetch_or(p + i, (u8)0, __ATOMIC_RELAXED);
+    if (n) __atomic_fetch_or(p + n - 1, (u8)0, __ATOMIC_RELAXED);
+}
+
 // KGBWT_PLAIN=1 in the environment makes the drop-in and batch calls use the plain path (debugging aid).
 static uint32_t env_flags() {
     static int plain = -1;
@@ -158,20 +180,35 @@ int run_fwd_jobs(Worker &C, kgbwt_fwd_job *jobs, int32_t count, uint32_t flags) 
     if (cudaMemsetAsync(E.text() + E.total(), 0, 64, s) != cudaSuccess)
         return fail(record_cuda_error(cudaGetLastError(), "cudaMemsetAsync", __FILE__, __LINE__));
     if ((rc = E.run(s, !(flags & KGBWT_PLAIN)))) return fail(rc);
-    // sampled indexes first (small); then each block's L column without its sentinel row: straight into the
-    // caller's U when every U is page-locked (two device-to-host copies per block), else through one copy into pinned
-    // staging and host copies (device-to-host copies into pageable memory are staged by the CUDA driver, block by block)
-    bool direct = true;
-    for (size_t k = 0; k < dev.size() && direct; k++) direct = page_locked(jobs[dev[k]].U);
-    if (!direct) {
-        const size_t lbytes = E.total() + dev.size();
-        if ((rc = C.stage_L.need(lbytes))) return fail(rc);
-        if (cudaMemcpyAsync(C.stage_L.p, E.lcol(), lbytes, cudaMemcpyDeviceToHost, s) != cudaSuccess)
-            return fail(record_cuda_error(cudaGetLastError(), "cudaMemcpyAsync(L)", __FILE__, __LINE__));
+    // sampled indexes first (small), with the L columns of short blocks for pageable buffers; then the other blocks' L
+    // columns without their sentinel rows, straight into the caller's U (two copies each)
+    std::vector<u8> direct(dev.size());
+    size_t staged = 0;
+    for (size_t k = 0; k < dev.size(); k++) {
+        direct[k] = page_locked(jobs[dev[k]].U) ? D_LOCKED : n[k] >= DIRECT_MIN ? D_PAGEABLE : D_STAGED;
+        if (!direct[k]) staged += n[k] + 1;
+    }
+    if (staged) {
+        if ((rc = C.stage_L.need(staged))) return fail(rc);
+        if (staged == E.total() + dev.size()) {  // all of them: the columns are contiguous
+            if (cudaMemcpyAsync(C.stage_L.p, E.lcol(), staged, cudaMemcpyDeviceToHost, s) != cudaSuccess)
+                return fail(record_cuda_error(cudaGetLastError(), "cudaMemcpyAsync(L)", __FILE__, __LINE__));
+        } else {
+            size_t at = 0;
+            for (size_t k = 0; k < dev.size(); k++) {
+                if (direct[k]) continue;
+                if (cudaMemcpyAsync(C.stage_L.p + at, E.lcol() + E.offsets()[k] + k, (size_t)n[k] + 1,
+                                    cudaMemcpyDeviceToHost, s) != cudaSuccess)
+                    return fail(record_cuda_error(cudaGetLastError(), "cudaMemcpyAsync(L)", __FILE__, __LINE__));
+                at += (size_t)n[k] + 1;
+            }
+        }
     }
     if ((rc = C.stage_I.need((size_t)E.samples() * 4))) return fail(rc);
     if (cudaMemcpyAsync(C.stage_I.p, E.samples_dev(), (size_t)E.samples() * 4, cudaMemcpyDeviceToHost, s) != cudaSuccess)
         return fail(record_cuda_error(cudaGetLastError(), "cudaMemcpyAsync(samples)", __FILE__, __LINE__));
+    for (size_t k = 0; k < dev.size(); k++)
+        if (direct[k] == D_PAGEABLE) touch_pages(jobs[dev[k]].U, n[k]);
     u32 err = 0;
     if ((rc = E.error_flag(s, &err))) return fail(rc);
     if (err) {
@@ -181,22 +218,21 @@ int run_fwd_jobs(Worker &C, kgbwt_fwd_job *jobs, int32_t count, uint32_t flags) 
         return fail(-2);
     }
     const u32 *I = reinterpret_cast<const u32 *>(C.stage_I.p);
-    for (size_t k = 0; k < dev.size() && !direct; k++) {
+    const u8 *SL = C.stage_L.p;
+    for (size_t k = 0; k < dev.size(); k++) {
         kgbwt_fwd_job &j = jobs[dev[k]];
-        const u8 *L = C.stage_L.p + E.offsets()[k] + k;
         const u32 p0 = I[E.iouts()[k]];
         if (p0 < 1 || p0 > (u32)j.n) return fail(-2);
-        memcpy(j.U, L, p0);
-        memcpy(j.U + p0, L + p0 + 1, (size_t)j.n - p0);
-    }
-    for (size_t k = 0; k < dev.size() && direct; k++) {
-        kgbwt_fwd_job &j = jobs[dev[k]];
+        if (!direct[k]) {
+            memcpy(j.U, SL, p0);
+            memcpy(j.U + p0, SL + p0 + 1, (size_t)j.n - p0);
+            SL += (size_t)j.n + 1;
+            continue;
+        }
         const u8 *L = E.lcol() + E.offsets()[k] + k;
-        const u32 p0 = I[E.iouts()[k]];
-        if (p0 < 1 || p0 > (u32)j.n) return fail(-2);
-        if ((p0 && cudaMemcpyAsync(j.U, L, p0, cudaMemcpyDeviceToHost, s) != cudaSuccess) ||
-            ((u32)j.n > p0 && cudaMemcpyAsync(j.U + p0, L + p0 + 1, (size_t)j.n - p0, cudaMemcpyDeviceToHost, s) !=
-                                 cudaSuccess))
+        if (cudaMemcpyAsync(j.U, L, p0, cudaMemcpyDeviceToHost, s) != cudaSuccess ||
+            ((u32)j.n > p0 &&
+             cudaMemcpyAsync(j.U + p0, L + p0 + 1, (size_t)j.n - p0, cudaMemcpyDeviceToHost, s) != cudaSuccess))
             return fail(record_cuda_error(cudaGetLastError(), "cudaMemcpyAsync(result)", __FILE__, __LINE__));
     }
     if (cudaStreamSynchronize(s) != cudaSuccess)
@@ -242,26 +278,47 @@ int run_inv_jobs(Worker &C, kgbwt_inv_job *jobs, int32_t count, uint32_t flags) 
         if (cudaMemcpyAsync(E.input() + E.offsets()[k], jobs[dev[k]].T, n[k], cudaMemcpyHostToDevice, s) != cudaSuccess)
             return fail(record_cuda_error(cudaGetLastError(), "cudaMemcpyAsync(bwt)", __FILE__, __LINE__));
     if ((rc = E.run(s, !(flags & KGBWT_PLAIN)))) return fail(rc);
-    // the decoded texts: straight into the callers' buffers when all are page-locked, else through pinned staging
-    bool direct = true;
-    for (size_t k = 0; k < dev.size() && direct; k++) direct = page_locked(jobs[dev[k]].U);
-    if (!direct) {
-        if ((rc = C.stage_L.need(E.total()))) return fail(rc);
-        if (cudaMemcpyAsync(C.stage_L.p, E.output(), E.total(), cudaMemcpyDeviceToHost, s) != cudaSuccess)
-            return fail(record_cuda_error(cudaGetLastError(), "cudaMemcpyAsync(text)", __FILE__, __LINE__));
+    // the decoded texts: short blocks for pageable buffers through pinned staging, the others straight into the
+    // callers' buffers once their status is known (a string that is no BWT leaves its buffer alone)
+    std::vector<u8> direct(dev.size());
+    size_t staged = 0;
+    for (size_t k = 0; k < dev.size(); k++) {
+        direct[k] = page_locked(jobs[dev[k]].U) ? D_LOCKED : n[k] >= DIRECT_MIN ? D_PAGEABLE : D_STAGED;
+        if (!direct[k]) staged += ((size_t)n[k] + 15) / 16 * 16;
     }
+    if (staged) {
+        if ((rc = C.stage_L.need(staged))) return fail(rc);
+        size_t at = 0;
+        if (staged == E.total()) {  // all of them: one copy (the engine's offsets are multiples of 16 too)
+            if (cudaMemcpyAsync(C.stage_L.p, E.output(), staged, cudaMemcpyDeviceToHost, s) != cudaSuccess)
+                return fail(record_cuda_error(cudaGetLastError(), "cudaMemcpyAsync(text)", __FILE__, __LINE__));
+            at = staged;
+        }
+        for (size_t k = 0; k < dev.size() && at < staged; k++) {
+            if (direct[k]) continue;
+            if (cudaMemcpyAsync(C.stage_L.p + at, E.output() + E.offsets()[k], n[k], cudaMemcpyDeviceToHost, s) !=
+                cudaSuccess)
+                return fail(record_cuda_error(cudaGetLastError(), "cudaMemcpyAsync(text)", __FILE__, __LINE__));
+            at += ((size_t)n[k] + 15) / 16 * 16;
+        }
+    }
+    for (size_t k = 0; k < dev.size(); k++)
+        if (direct[k] == D_PAGEABLE) touch_pages(jobs[dev[k]].U, n[k]);
     std::vector<int> st;
     if ((rc = E.fetch_status(s, st))) return fail(rc);
     int first = 0;
+    const u8 *SL = C.stage_L.p;
     for (size_t k = 0; k < dev.size(); k++) {
         kgbwt_inv_job &j = jobs[dev[k]];
+        const u8 *src = SL;
+        if (!direct[k]) SL += ((size_t)n[k] + 15) / 16 * 16;
         if (st[k]) {
             j.rc = -1;
             if (!first) { first = -1; record_error("inverse BWT: not a valid BWT string for its primary index"); }
             continue;
         }
-        if (!direct) {
-            memcpy(j.U, C.stage_L.p + E.offsets()[k], (size_t)j.n);
+        if (!direct[k]) {
+            memcpy(j.U, src, (size_t)j.n);
             continue;
         }
         if (cudaMemcpyAsync(j.U, E.output() + E.offsets()[k], (size_t)j.n, cudaMemcpyDeviceToHost, s) != cudaSuccess)
@@ -615,6 +672,7 @@ int32_t kgbwt_engine_fwd(kgbwt_engine *e, const uint8_t *dT, uint8_t *dL, int32_
         if (blocks[b].n < 2 || bad_r((int32_t)blocks[b].r) || blocks[b].n > 0x7FFFFFFFu) return -1;
         off[b] = blocks[b].off; n[b] = blocks[b].n; r[b] = blocks[b].r; io[b] = blocks[b].iout;
     }
+    if (int rc = refuse_capture((cudaStream_t)stream)) return rc;
     int rc = e->fwd.plan_external(off.data(), n.data(), r.data(), io.data(), count, const_cast<uint8_t *>(dT), dL,
                                   reinterpret_cast<u32 *>(dI), reinterpret_cast<u32 *>(dSA));
     if (rc) return rc;
@@ -632,6 +690,7 @@ int32_t kgbwt_engine_inv(kgbwt_engine *e, const uint8_t *dU, uint8_t *dOut, cons
         if (blocks[b].n < 2 || blocks[b].p0 < 1 || blocks[b].p0 > blocks[b].n || blocks[b].n > 0x7FFFFFFFu) return -1;
         off[b] = blocks[b].off; n[b] = blocks[b].n; p0[b] = blocks[b].p0;
     }
+    if (int rc = refuse_capture((cudaStream_t)stream)) return rc;
     int rc = e->inv.plan_external(off.data(), n.data(), p0.data(), count, const_cast<uint8_t *>(dU), dOut);
     if (rc) return rc;
     e->last = (cudaStream_t)stream;

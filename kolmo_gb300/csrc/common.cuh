@@ -16,6 +16,8 @@ typedef unsigned long long u64;
 // enclosing function return the C-ABI code (-2 for resources and device errors).
 int record_cuda_error(cudaError_t e, const char *what, const char *file, int line);
 void record_error(const char *msg);
+// -2 (with the error recorded) when `s` is being captured: the engines upload from host memory they reuse.
+int refuse_capture(cudaStream_t s);
 #define KGB_CHECK(x)                                                                         \
     do {                                                                                     \
         cudaError_t e__ = (x);                                                               \

@@ -1838,6 +1838,10 @@ FwdEngine::~FwdEngine() { free_all(); }
 void FwdEngine::free_all() {
     if (cap_stream) cudaStreamDestroy(cap_stream);
     cap_stream = nullptr;
+    if (up_pending) cudaEventSynchronize(up_done);
+    if (up_done) cudaEventDestroy(up_done);
+    up_done = nullptr;
+    up_pending = false;
     if (gexec) cudaGraphExecDestroy(gexec);
     if (graph) cudaGraphDestroy(graph);
     gexec = nullptr;
@@ -2089,19 +2093,47 @@ static int ceil_log2(u64 x) { int k = 0; while ((1ull << k) < x) k++; return k; 
 bool FwdEngine::lsd_enabled() const { return cfg.lsd_round0 && N < (1ull << 30); }
 
 int FwdEngine::setup_round0(cudaStream_t s) {
-    // block table, round-0 lists and their tile maps are laid out on the host (B entries, small)
-    const u32 smax = (u32)cfg.tile_cap / 2;
-    std::vector<BlockInfo> bi(B);
+    // the block table and the control block (the LSD round 0 needs no more), uploaded without waiting for the stream:
+    // their sources are members that the next call changes only once these copies are done
+    if (up_pending) {
+        up_pending = false;
+        KGB_CHECK(cudaEventSynchronize(up_done));
+    }
+    if (!up_done) KGB_CHECK(cudaEventCreateWithFlags(&up_done, cudaEventDisableTiming));
+    h_bi.resize(B);
     u32 soff_b = 0, lt_b = 0;
+    for (u32 b = 0; b < B; b++) {
+        h_bi[b] = BlockInfo{h_off[b], h_n[b], h_r[b], h_iout[b], soff_b, lt_b};
+        soff_b += h_n[b];
+        lt_b += (h_n[b] + LSD_TILE - 1) / LSD_TILE;
+    }
+    Ctl &c = h_c0;
+    memset(&c, 0, sizeof(c));
+    c.maxrounds = (u32)ceil_log2(maxn) + 3;
+    c.seq = ++call_seq;
+    c.h0 = 8;  // the tile path's prefix; the LSD round 0 sets its own
+    c.lsd_tiles = lt_b;
+    c.idn = (u32)N;  // N is the batch's extent: max over blocks of off + n
+    if (cfg.warp_path)  // (the stamps tell the block kernel's tiles from the warp kernel's)
+        for (int l : {(int)L_S0, (int)L_S1, (int)L_KS}) KGB_CHECK(cudaMemsetAsync(lists[l].tbig, 0xFF, cap_tms * 4, s));
+    if (!lsd_enabled())
+        if (int rc = setup_tile_round0(s)) return rc;
+    KGB_CHECK(cudaMemcpyAsync(d_blk, h_bi.data(), B * sizeof(BlockInfo), cudaMemcpyHostToDevice, s));
+    KGB_CHECK(cudaMemcpyAsync(d_ctl, &h_c0, sizeof(Ctl), cudaMemcpyHostToDevice, s));
+    KGB_CHECK(cudaEventRecord(up_done, s));
+    up_pending = true;
+    return 0;
+}
+
+// The tile path's round 0: lists and tile maps laid out on the host (B entries, small).
+int FwdEngine::setup_tile_round0(cudaStream_t s) {
+    const u32 smax = (u32)cfg.tile_cap / 2;
     std::vector<u32> lstart(B);
     std::vector<u8> large(B);
     std::vector<Seg> seg_s, seg_l;
     std::vector<u32> tm_s, tm_l, big_s;
     u64 es = 0, el = 0;
     for (u32 b = 0; b < B; b++) {
-        bi[b] = BlockInfo{h_off[b], h_n[b], h_r[b], h_iout[b], soff_b, lt_b};
-        soff_b += h_n[b];
-        lt_b += (h_n[b] + LSD_TILE - 1) / LSD_TILE;
         large[b] = h_n[b] > smax;
         Seg g;
         g.len = h_n[b]; g.head = 0; g.bd = b;
@@ -2119,19 +2151,9 @@ int FwdEngine::setup_round0(cudaStream_t s) {
             es += h_n[b];
         }
     }
-    // staging: the small vectors go through one pinned buffer
-    Ctl c;
-    memset(&c, 0, sizeof(c));
-    c.cnt[L_S0] = ((u64)seg_s.size() << 32) | es;
-    c.cnt[L_L0] = ((u64)seg_l.size() << 32) | el;
-    c.maxrounds = (u32)ceil_log2(maxn) + 3;
-    c.seq = ++call_seq;
-    c.h0 = 8;  // the tile path's prefix; the LSD round 0 sets its own
-    c.lsd_tiles = lt_b;
-    c.idn = (u32)N;  // N is the batch's extent: max over blocks of off + n
-    KGB_CHECK(cudaMemcpyAsync(d_blk, bi.data(), B * sizeof(BlockInfo), cudaMemcpyHostToDevice, s));
-    const size_t ntm = cap_tms;
-    for (int l : {(int)L_S0, (int)L_S1, (int)L_KS}) KGB_CHECK(cudaMemsetAsync(lists[l].tbig, 0xFF, ntm * 4, s));
+    h_c0.cnt[L_S0] = ((u64)seg_s.size() << 32) | es;
+    h_c0.cnt[L_L0] = ((u64)seg_l.size() << 32) | el;
+    for (int l : {(int)L_S0, (int)L_S1, (int)L_KS}) KGB_CHECK(cudaMemsetAsync(lists[l].tbig, 0xFF, cap_tms * 4, s));
     if (!seg_s.empty()) {
         KGB_CHECK(cudaMemcpyAsync(lists[L_S0].seg, seg_s.data(), seg_s.size() * sizeof(Seg), cudaMemcpyHostToDevice, s));
         if (!tm_s.empty()) KGB_CHECK(cudaMemcpyAsync(lists[L_S0].tmap, tm_s.data(), tm_s.size() * 4, cudaMemcpyHostToDevice, s));
@@ -2145,8 +2167,6 @@ int FwdEngine::setup_round0(cudaStream_t s) {
         KGB_CHECK(cudaMemcpyAsync(lists[L_L0].seg, seg_l.data(), seg_l.size() * sizeof(Seg), cudaMemcpyHostToDevice, s));
         KGB_CHECK(cudaMemcpyAsync(lists[L_L0].tmap, tm_l.data(), tm_l.size() * 4, cudaMemcpyHostToDevice, s));
     }
-    *h_ctl = c;
-    KGB_CHECK(cudaMemcpyAsync(d_ctl, h_ctl, sizeof(Ctl), cudaMemcpyHostToDevice, s));
     // per-block list starts and classes: stored behind the block table in the histogram rows, which are zero
     // outside a bucket pass and are restored to zero by k_init's caller below
     u32 *d_lstart = d_cursor;

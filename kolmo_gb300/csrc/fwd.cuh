@@ -140,6 +140,7 @@ class FwdEngine {
     int build_graph(cudaStream_t s);
     void free_all();
     int setup_round0(cudaStream_t s);
+    int setup_tile_round0(cudaStream_t s);
     void set_caps(FwdArgs &a) const;
     bool lsd_enabled() const;
     u32 call_seq = 0;
@@ -178,6 +179,10 @@ class FwdEngine {
     u8 *d_dest = nullptr;
     Ctl *d_ctl = nullptr;
     Ctl *h_ctl = nullptr;  // pinned mirror
+    std::vector<BlockInfo> h_bi;  // sources of the uploads in flight: left alone until up_done
+    Ctl h_c0{};
+    cudaEvent_t up_done = nullptr;
+    bool up_pending = false;
     void *pool = nullptr;
     size_t pool_bytes = 0;
 

@@ -54,7 +54,6 @@ struct InvArgs {
     u8 *out;
     u32 *psi;
     u32 *csum;
-    const u32 *cblk;
     u32 *C;
     u16 *ft;  // per block: FT entries, lowest byte value | highest << 8
     const InvBlock *blk;
@@ -100,12 +99,22 @@ __device__ __forceinline__ u32 f_search(const u32 *Cs, u32 row, u32 lo, u32 hi) 
     return lo;
 }
 
+// The block of psi-build chunk q: the last one whose first chunk is <= q.
+__device__ __forceinline__ u32 chunk_block(const InvArgs &a, u64 q) {
+    u32 lo = 0, hi = a.B - 1;
+    while (lo < hi) {
+        const u32 mid = (lo + hi + 1) >> 1;
+        if (__ldg(&a.blk[mid].chunk_base) <= q) lo = mid; else hi = mid - 1;
+    }
+    return lo;
+}
+
 // Per-chunk byte histograms (a chunk is chunkt consecutive tiles of one block).
 __global__ void __launch_bounds__(ITPB) k_inv_chunkhist(InvArgs a) {
     __shared__ u32 h[256];
     const u32 lane = lane_id();
     for (u64 q = blockIdx.x; q < a.nchunk_all; q += gridDim.x) {
-        const InvBlock B = a.blk[a.cblk[q]];
+        const InvBlock B = a.blk[chunk_block(a, q)];
         const u32 start = (u32)(q - B.chunk_base) * (ITILE * a.chunkt);
         const u32 cnt = min(ITILE * a.chunkt, B.n - start);
         const u8 *src = a.U + (u64)B.off + start;
@@ -201,7 +210,7 @@ __global__ void __launch_bounds__(ITPB, 3) k_inv_scatter(InvArgs a) {
     const u32 lane = lane_id(), warp = warp_id();
     for (int i = threadIdx.x; i < NW * 256 * RQ; i += ITPB) (&mask[0][0])[i] = 0;
     for (u64 q = blockIdx.x; q < a.nchunk_all; q += gridDim.x) {
-        const u32 b = a.cblk[q];
+        const u32 b = chunk_block(a, q);
         const InvBlock B = a.blk[b];
         const u32 cstart = (u32)(q - B.chunk_base) * (ITILE * a.chunkt);
         const u32 ccnt = min(ITILE * a.chunkt, B.n - cstart);
@@ -442,6 +451,10 @@ InvEngine::InvEngine() {}
 InvEngine::~InvEngine() { free_all(); }
 
 void InvEngine::free_all() {
+    if (up_pending) cudaEventSynchronize(up_done);
+    if (up_done) cudaEventDestroy(up_done);
+    up_done = nullptr;
+    up_pending = false;
     if (cap_stream) cudaStreamDestroy(cap_stream);
     cap_stream = nullptr;
     if (gexec) cudaGraphExecDestroy(gexec);
@@ -461,7 +474,6 @@ void InvEngine::layout(u64 ncap, u32 bcap, u64 tcap, u64 ccap, Add add) {
     add((void **)&own_out, ncap + 64);
     add((void **)&d_psi, (ncap + bcap + 16) * 4);
     add((void **)&d_csum, tcap * 256 * 4);
-    add((void **)&d_cblk, tcap * 4);
     add((void **)&d_C, (size_t)bcap * 257 * 4);
     add((void **)&d_ft, (size_t)bcap * FT * 2);
     add((void **)&d_blk, (size_t)bcap * sizeof(InvBlock));
@@ -519,12 +531,11 @@ static u32 mark_of(const u32 *n, int count) {
 }
 
 static int plan_layout(const u32 *off, const u32 *n, const u32 *p0, int count, std::vector<InvBlock> &blk,
-                       std::vector<u32> &cblk, u64 &nchunk_all, u64 &nchains, u32 &chunkt,
+                       u64 &nchunk_all, u64 &nchains, u32 &chunkt,
                        u32 &nwalk) {
     blk.resize(count);
     nwalk = 0;
     const u32 mark = mark_of(n, count);
-    cblk.clear();
     nchunk_all = 0; nchains = 0;
     auto chunks_of = [&](u32 t) {
         u64 c = 0;
@@ -544,7 +555,6 @@ static int plan_layout(const u32 *off, const u32 *n, const u32 *p0, int count, s
         B.chain_cap = B.nreg + 1 + n[b] / CAPC + 4;
         B.qbase = nwalk;
         nwalk += B.nreg + 1;
-        for (u32 t = 0; t < B.nchunk; t++) cblk.push_back((u32)b);
         nchunk_all += B.nchunk;
         nchains += B.chain_cap;
         blk[b] = B;
@@ -558,10 +568,9 @@ u64 InvEngine::estimate_bytes(const u32 *n, int count) {
     u64 o = 0;
     for (int b = 0; b < count; b++) { off[b] = (u32)o; o += ((u64)n[b] + 15) / 16 * 16; }
     std::vector<InvBlock> blk;
-    std::vector<u32> cblk;
     u64 nch = 0, nchains_ = 0;
     u32 ct = 0, nw = 0;
-    if (plan_layout(off.data(), n, p0.data(), count, blk, cblk, nch, nchains_, ct, nw)) return ~0ull;
+    if (plan_layout(off.data(), n, p0.data(), count, blk, nch, nchains_, ct, nw)) return ~0ull;
     u64 total = 0;
     layout(std::max<u64>(o, Ncap), std::max<u32>((u32)count, Bcap), std::max<u64>(nch, Tcap),
            std::max<u64>(nchains_, Ccap),
@@ -569,8 +578,17 @@ u64 InvEngine::estimate_bytes(const u32 *n, int count) {
     return total;
 }
 
+// The block table's upload of the call before: its source is changed only once it is done.
+int InvEngine::uploads_done() {
+    if (!up_pending) return 0;
+    up_pending = false;
+    KGB_CHECK(cudaEventSynchronize(up_done));
+    return 0;
+}
+
 int InvEngine::plan(const u32 *n, const u32 *p0, int count) {
     if (count <= 0) return -1;
+    if (int rc = uploads_done()) return rc;
     h_off.resize(count);
     u64 off = 0;
     for (int b = 0; b < count; b++) {
@@ -578,22 +596,20 @@ int InvEngine::plan(const u32 *n, const u32 *p0, int count) {
         off += ((u64)n[b] + 15) / 16 * 16;
         if (off > 0xFFFF0000ull) return -1;
     }
-    std::vector<u32> cblk;
-    if (plan_layout(h_off.data(), n, p0, count, h_blk, cblk, nchunk_all, nchains, chunkt, nwalk)) return -1;
+    if (plan_layout(h_off.data(), n, p0, count, h_blk, nchunk_all, nchains, chunkt, nwalk)) return -1;
     N = off; B = (u32)count;
     int rc = grow(N, B, nchunk_all, nchains);
     if (rc) return rc;
     ext = false;
     d_U = own_U; d_out = own_out;
-    KGB_CHECK(cudaMemcpy(d_cblk, cblk.data(), cblk.size() * 4, cudaMemcpyHostToDevice));
     return 0;
 }
 
 int InvEngine::plan_external(const u32 *off, const u32 *n, const u32 *p0, int count, u8 *dU, u8 *dOut) {
     if (count <= 0) return -1;
+    if (int rc = uploads_done()) return rc;
     h_off.assign(off, off + count);
-    std::vector<u32> cblk;
-    if (plan_layout(off, n, p0, count, h_blk, cblk, nchunk_all, nchains, chunkt, nwalk)) return -1;
+    if (plan_layout(off, n, p0, count, h_blk, nchunk_all, nchains, chunkt, nwalk)) return -1;
     u64 end = 0;
     for (int b = 0; b < count; b++) end = std::max<u64>(end, (u64)off[b] + n[b]);
     N = end; B = (u32)count;
@@ -601,7 +617,6 @@ int InvEngine::plan_external(const u32 *off, const u32 *n, const u32 *p0, int co
     if (rc) return rc;
     ext = true;
     d_U = dU; d_out = dOut;
-    KGB_CHECK(cudaMemcpy(d_cblk, cblk.data(), cblk.size() * 4, cudaMemcpyHostToDevice));
     return 0;
 }
 
@@ -614,7 +629,7 @@ u32 InvEngine::nmax() const {
 int InvEngine::enqueue(cudaStream_t s, long long *launches) {
     InvArgs a;
     memset(&a, 0, sizeof(a));
-    a.U = d_U; a.out = d_out; a.psi = d_psi; a.csum = d_csum; a.cblk = d_cblk; a.C = d_C; a.ft = d_ft; a.blk = d_blk; a.B = B;
+    a.U = d_U; a.out = d_out; a.psi = d_psi; a.csum = d_csum; a.C = d_C; a.ft = d_ft; a.blk = d_blk; a.B = B;
     a.nchunk_all = nchunk_all; a.chunkt = chunkt; a.nchains = nchains; a.len = d_len; a.pair = d_pair; a.dyn = d_dyn;
     a.status = d_status; a.buf = d_buf; a.nwalk = nwalk; a.cap_n = Ncap;
     a.nmax = nmax();
@@ -648,6 +663,7 @@ int InvEngine::enqueue(cudaStream_t s, long long *launches) {
 
 int InvEngine::run(cudaStream_t s, bool use_graph) {
     stats = InvStats{};
+    if (!up_done) KGB_CHECK(cudaEventCreateWithFlags(&up_done, cudaEventDisableTiming));
     if (!sm_count) {
         int dev;
         KGB_CHECK(cudaGetDevice(&dev));
@@ -656,7 +672,8 @@ int InvEngine::run(cudaStream_t s, bool use_graph) {
     }
     stats.jumps = 1;
     KGB_CHECK(cudaMemcpyAsync(d_blk, h_blk.data(), h_blk.size() * sizeof(InvBlock), cudaMemcpyHostToDevice, s));
-    KGB_CHECK(cudaStreamSynchronize(s));  // host vectors are pageable: finish before they can change
+    KGB_CHECK(cudaEventRecord(up_done, s));
+    up_pending = true;
     prof.reset();
     prof_run = !use_graph && prof.on;
     if (!use_graph) return enqueue(s, &stats.launches);
@@ -714,7 +731,6 @@ struct NoAllocScratch {
     u32 csum[NA_CHUNKS * 256];
     u32 C[264];
     u16 ft[FT];
-    u32 cblk[NA_CHUNKS];
     InvBlock blk[1];
     u64 pair[NA_CHAINS];
     u32 len[NA_CHAINS];
@@ -747,15 +763,13 @@ static int unbwt_noalloc(const u8 *dU, u8 *dT, u32 n, u32 p0, cudaStream_t s) {
     int rc = 0;
     NoAllocScratch *S = noalloc_scratch(&rc);
     if (!S) return rc;
-    // host-side tables on the stack: one block and its chunk map
+    // the block's table entry, on the stack
     InvBlock B;
     B.off = 0; B.n = n; B.p0 = p0;
     B.chunk_base = 0; B.nchunk = (n + ITILE - 1) / ITILE;
     B.nreg = n / MARK; B.chain_base = 0; B.chain_cap = B.nreg + 1 + n / CAPC + 4; B.qbase = 0;
     mark_params(B);
-    u32 cblk[NA_CHUNKS] = {0};
     KGB_CHECK(cudaMemcpyAsync(S->blk, &B, sizeof(B), cudaMemcpyHostToDevice, s));
-    KGB_CHECK(cudaMemcpyAsync(S->cblk, cblk, sizeof(u32) * B.nchunk, cudaMemcpyHostToDevice, s));
     // the array keeps the previous call's contents: reset what must start at zero (or at "no successor")
     KGB_CHECK(cudaMemsetAsync(S->len, 0, sizeof(u32) * B.chain_cap, s));
     KGB_CHECK(cudaMemsetAsync(S->pair, 0xFF, sizeof(u64) * B.chain_cap, s));
@@ -763,7 +777,7 @@ static int unbwt_noalloc(const u8 *dU, u8 *dT, u32 n, u32 p0, cudaStream_t s) {
     KGB_CHECK(cudaMemsetAsync(S->status, 0, sizeof(S->status), s));
     InvArgs a;
     memset(&a, 0, sizeof(a));
-    a.U = dU; a.out = dT; a.psi = S->psi; a.csum = S->csum; a.cblk = S->cblk; a.C = S->C; a.ft = S->ft; a.blk = S->blk; a.B = 1;
+    a.U = dU; a.out = dT; a.psi = S->psi; a.csum = S->csum; a.C = S->C; a.ft = S->ft; a.blk = S->blk; a.B = 1;
     a.nchunk_all = B.nchunk; a.chunkt = 1; a.nchains = B.chain_cap; a.len = S->len; a.pair = S->pair; a.dyn = S->dyn;
     a.status = S->status; a.buf = S->buf; a.nwalk = B.nreg + 1; a.cap_n = n; a.nmax = n;
     k_inv_chunkhist<<<B.nchunk, ITPB, 0, s>>>(a);

@@ -54,6 +54,7 @@ class InvEngine {
     int build_graph(cudaStream_t s);
     int enqueue(cudaStream_t s, long long *launches);
     u32 nmax() const;
+    int uploads_done();
     void free_all();
     u64 Ncap = 0, Tcap = 0, Ccap = 0;
     u32 Bcap = 0;
@@ -61,10 +62,12 @@ class InvEngine {
     u32 B = 0, chunkt = 0, nwalk = 0;
     int walk_grid = 0;   // resident CTAs of the walk kernel
     std::vector<u32> h_off;
-    std::vector<InvBlock> h_blk;
+    std::vector<InvBlock> h_blk;  // source of the table's upload: left alone until up_done
+    cudaEvent_t up_done = nullptr;
+    bool up_pending = false;
     bool ext = false;
     u8 *d_U = nullptr, *d_out = nullptr, *own_U = nullptr, *own_out = nullptr;
-    u32 *d_psi = nullptr, *d_csum = nullptr, *d_C = nullptr, *d_cblk = nullptr;
+    u32 *d_psi = nullptr, *d_csum = nullptr, *d_C = nullptr;
     u32 *d_len = nullptr;
     u64 *d_pair = nullptr;
     u32 *d_dyn = nullptr, *d_status = nullptr;
