@@ -33,11 +33,11 @@ constexpr u64 ST_AGG = 1ull << 30, ST_PRE = 2ull << 30, ST_VAL = (1ull << 30) - 
 constexpr u64 ST_EPOCH = 0xFFFFFFFF00000000ull;
 constexpr int LB_WIN = 8;  // look-back window (predecessor words read per step)
 
-// Which keys: the tuning table's choice per batch size, by measurement. Coded keys halve the passes, compare more in the
-// segmentation and leave slightly larger groups. Forward call, coded against the best raw width: 1 MiB Markov block
-// 0.24 ms against 0.29, ACGT 0.24 and 0.28, log lines 0.52 and 0.52, prose 0.73 and 0.72; 16 MiB 1.73 and 2.24, 1.69 and
-// 2.24, 3.14 and 3.37, 3.68 and 3.85; mixed batch of 64 blocks (216 MB) 28.9 and 34.3. Between 32 and 128 MiB the table
-// keeps raw 16 bytes for the sake of prose (64 MiB: 15.5 against 15.7).
+// Which keys: the tuning table's choice per batch size, by measurement; it takes coded keys throughout. They halve the
+// passes, compare more in the segmentation and leave slightly larger groups. Forward call, coded against raw 16 bytes:
+// log lines 20 KB 0.20 ms against 0.22, 1 MiB 0.41 and 0.44, 30 MB 5.65 and 5.95; prose 1 MiB 0.49 and 0.55, 64 slices of
+// 512 KiB 4.18 and 5.34, 64 MiB 14.48 and 14.70; 48 MiB Markov 5.39 and 7.90; 16 mixed blocks (53 MB) 8.00 and 11.17.
+// Raw keys stay for engines that ask for 12 or 16 bytes and where no table is loaded.
 __host__ __device__ __forceinline__ bool lsd_coded(const FwdArgs &a) { return a.lsd_bytes == 8; }
 __device__ __forceinline__ u32 active_slots(const Ctl *c) { return c->lsd_act; }  // bit s: slot s varies
 
