@@ -3,6 +3,8 @@
 #include "kgbwt.h"
 
 #include <dlfcn.h>
+#include <sys/mman.h>
+#include <unistd.h>
 
 #include <algorithm>
 #include <cstdio>
@@ -142,6 +144,18 @@ static void touch_pages(u8 *p, size_t n) {
     if (n) __atomic_fetch_or(p + n - 1, (u8)0, __ATOMIC_RELAXED);
 }
 
+// Whether every page of the buffer is mapped (false also where the system does not say).
+static bool pages_mapped(const u8 *p, size_t n) {
+    const size_t ps = (size_t)sysconf(_SC_PAGESIZE);
+    const uintptr_t b = (uintptr_t)p & ~(uintptr_t)(ps - 1);
+    const size_t len = (uintptr_t)p + n - b;
+    std::vector<unsigned char> in((len + ps - 1) / ps);
+    if (mincore((void *)b, len, in.data())) return false;
+    for (unsigned char c : in)
+        if (!(c & 1)) return false;
+    return true;
+}
+
 // KGBWT_PLAIN=1 in the environment makes the drop-in and batch calls use the plain path (debugging aid).
 static uint32_t env_flags() {
     static int plain = -1;
@@ -278,12 +292,15 @@ int run_inv_jobs(Worker &C, kgbwt_inv_job *jobs, int32_t count, uint32_t flags) 
         if (cudaMemcpyAsync(E.input() + E.offsets()[k], jobs[dev[k]].T, n[k], cudaMemcpyHostToDevice, s) != cudaSuccess)
             return fail(record_cuda_error(cudaGetLastError(), "cudaMemcpyAsync(bwt)", __FILE__, __LINE__));
     if ((rc = E.run(s, !(flags & KGBWT_PLAIN)))) return fail(rc);
-    // the decoded texts: short blocks for pageable buffers through pinned staging, the others straight into the
-    // callers' buffers once their status is known (a string that is no BWT leaves its buffer alone)
+    // the decoded texts: short blocks for pageable buffers, and those whose buffers are not mapped yet (mapping 30 MB
+    // can take longer than decoding it, and the copy from staging does it in passing), through pinned staging; the
+    // others straight into the callers' buffers once their status is known (a string that is no BWT leaves its buffer
+    // alone)
     std::vector<u8> direct(dev.size());
     size_t staged = 0;
     for (size_t k = 0; k < dev.size(); k++) {
-        direct[k] = page_locked(jobs[dev[k]].U) ? D_LOCKED : n[k] >= DIRECT_MIN ? D_PAGEABLE : D_STAGED;
+        u8 *U = jobs[dev[k]].U;
+        direct[k] = page_locked(U) ? D_LOCKED : n[k] >= DIRECT_MIN && pages_mapped(U, n[k]) ? D_PAGEABLE : D_STAGED;
         if (!direct[k]) staged += ((size_t)n[k] + 15) / 16 * 16;
     }
     if (staged) {
@@ -302,8 +319,6 @@ int run_inv_jobs(Worker &C, kgbwt_inv_job *jobs, int32_t count, uint32_t flags) 
             at += ((size_t)n[k] + 15) / 16 * 16;
         }
     }
-    for (size_t k = 0; k < dev.size(); k++)
-        if (direct[k] == D_PAGEABLE) touch_pages(jobs[dev[k]].U, n[k]);
     std::vector<int> st;
     if ((rc = E.fetch_status(s, st))) return fail(rc);
     int first = 0;

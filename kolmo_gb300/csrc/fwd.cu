@@ -2426,14 +2426,20 @@ int FwdEngine::run_plain(cudaStream_t s) {
             if (!prefix) {
                 L.tag(K_FIXUP, cnt_e(L_R0 + (rp ^ 1)));
                 KGB_CHECK(L.go(k_fixup, grid_msd, TPB, 0, a));
+            }
+            // what the control block of the last read tells to be empty is not launched (nor read again): the key
+            // generation and the bucket passes without large groups, the tiles of an empty list
+            const bool large = cnt_e(L_L0 + rp) > 0;
+            if (large && !prefix) {
                 L.tag(K_KEYGEN, cnt_e(L_L0 + rp), cnt_s(L_L0 + rp));
                 KGB_CHECK(L.go(k_keygen, grid_msd, TPB, 0, a));
             }
-            L.tag(K_CTL, 0);
-            KGB_CHECK(L.go(k_ctl_msd_begin, 1, 1, 0, a));
-            if (int rc = read_ctl()) return rc;
-            u32 lin = L_L0 + h_ctl->rpar;
-            u32 more = cnt_e(lin) > 0;
+            if (large) {
+                L.tag(K_CTL, 0);
+                KGB_CHECK(L.go(k_ctl_msd_begin, 1, 1, 0, a));
+            }
+            u32 lin = L_L0 + rp;
+            u32 more = large;
             int pass = 0;
             while (more) {
                 prof.pass = pass++;
@@ -2454,6 +2460,7 @@ int FwdEngine::run_plain(cudaStream_t s) {
                 for (int keyed = 0; keyed < 2; keyed++) {
                     const u32 lid = keyed ? L_KS : L_S0 + h_ctl->rpar;
                     const u32 segs = cnt_s(lid);
+                    if (!segs) continue;
                     for (int wk = 0; wk < 2; wk++) {
                         if (wk && !cfg.warp_path) break;
                         const u64 before = h_ctl->tile_elems[wk];
@@ -2464,8 +2471,8 @@ int FwdEngine::run_plain(cudaStream_t s) {
                     }
                 }
             } else {
-                KGB_CHECK(enq_tile(L, a, prefix, false));
-                KGB_CHECK(enq_tile(L, a, prefix, true));
+                if (cnt_s(L_S0 + rp)) KGB_CHECK(enq_tile(L, a, prefix, false));
+                if (cnt_s(L_KS)) KGB_CHECK(enq_tile(L, a, prefix, true));
             }
             if (!prefix && cnt_e(L_M0 + rp)) {
                 L.tag(K_MKEYS, cnt_e(L_M0 + rp), cnt_s(L_M0 + rp));
