@@ -248,7 +248,7 @@ def single_blocks(workload: str, rank: int, mib: int):
 # case: profiles/traffic_group_thread_lsd_pass_prose16.md (tiny groups) and profiles/lsd_pass_prose16.md (the
 # round-0 radix pass, averaged over a 16-pass step). The 64 MiB launch's traffic is scaled by the suffixes it
 # processes.
-TRAFFIC_PER_SUFFIX = {"group_thread": 35.1, "lsd_pass": 13.9}
+TRAFFIC_PER_SUFFIX = {"group_thread": 35.1, "lsd_pass": 15.0}
 RANK_SORTERS = ("tile_sort_rank", "tile_warp_rank", "group_thread", "group_warp", "keygen")
 
 
@@ -426,6 +426,9 @@ def run_ours(args, world, rank, local):
         lc = eng.last_config()
         h0 = lc["lsd_bytes"] if lc["lsd_round0"] else 8  # prefix bytes round 0 sorts (the first rank round's h)
         bk, table = profile_table(prof_f, prof_i, n, h0, peak)
+        if lc["lsd_round0"] and lc["lsd_bytes"] == 8:  # coded keys: how far they reach depends on the group
+            for row in table[1:]:
+                row["h"] = None
         for k, d in bk.items():
             a = by_kernel.setdefault(k, {"launches": 0, "ms": 0.0, "bytes": 0.0, "elems": 0})
             for f in a:

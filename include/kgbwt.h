@@ -92,8 +92,9 @@ int32_t kgbwt_engine_config(kgbwt_engine *e, int32_t tile_cap, int32_t tile_ctas
  * KGBWT_OPT_WARP_PATH (0/1, default 1): tiles whose groups are all at most 32 long go to the warp-level kernel.
  * KGBWT_OPT_LSD_ROUND0 (0/1, default 1): the first round (all suffixes by their prefix) is one LSD radix sort of the
  *   whole batch; 0: bucket passes and tile kernels over 8-byte prefixes as in the later rounds.
- * KGBWT_OPT_LSD_BYTES (8, 12 or 16, default 16): prefix bytes that LSD round sorts (16 replaces the first rank round;
- *   the rank rounds then double from there).
+ * KGBWT_OPT_LSD_BYTES (8, 12 or 16, default 16): key bytes that LSD round sorts: 16 or 12, the suffix's first bytes
+ *   themselves; 8, the first 64 bits of the suffix in an order-preserving prefix code of its block's bytes (as many
+ *   characters as their codewords fit; the tuning table's choice). The rank rounds double from there.
  * KGBWT_OPT_CHAIN_FROM (0..64, default 1): from this rank round on, in rounds where doubling has stalled, a group of
  *   up to eight suffixes that doubling leaves whole is ordered along its repeat chain (the copies of a repeated
  *   stretch move through the rounds together and are ordered where the repeat ends) instead of waiting for the

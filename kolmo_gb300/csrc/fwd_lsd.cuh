@@ -31,7 +31,7 @@ constexpr int SEG_IPT = 16, SEG_TILE = TPB * SEG_IPT;  // positions per segmenta
 // epoch (an earlier slot or call) counts as not yet published
 constexpr u64 ST_AGG = 1ull << 30, ST_PRE = 2ull << 30, ST_VAL = (1ull << 30) - 1;
 constexpr u64 ST_EPOCH = 0xFFFFFFFF00000000ull;
-constexpr int LB_WIN = 8;  // look-back window (predecessor words read per step)
+constexpr int LB_WIN = 4;  // look-back window (predecessor words read per step; 8: 0.5% slower on 64 MiB of prose)
 
 // Which keys: the tuning table's choice per batch size, by measurement; it takes coded keys throughout. They halve the
 // passes, compare more in the segmentation and leave slightly larger groups. Forward call, coded against raw 16 bytes:
@@ -736,7 +736,7 @@ __global__ void __launch_bounds__(TPB, 3) k_seg_count(FwdArgs a) {
             for (int q = 0; q < QB; q++) {
                 const u32 p = cb + (j0 + q) * 32 + lane;
                 b[q] = p < v.m && br.x != br.y ? blk_of_pos(a, p, br.x, br.y) : br.x;
-                id[q] = p < v.m ? v.val[p] : bi0.off;
+                id[q] = p < v.m ? __ldcs(v.val + p) : bi0.off;
             }
 #pragma unroll
             for (int q = 0; q < QB; q++) {
@@ -789,7 +789,7 @@ __global__ void __launch_bounds__(TPB, 3) k_seg_count(FwdArgs a) {
                     // the L column of the sorted order so far: final for groups of one, overwritten for the others
                     const u8 c = id[q] == bi.off ? (u8)0 : tx[q].has_before ? tx[q].before : __ldg(a.T + id[q] - 1);
                     KGB_GUARD(p >= bi.soff && p - bi.soff < bi.n, &a.ctl->err, E_RANK)
-                    a.L[(u64)bi.off + b[q] + (p - bi.soff) + 1] = c;
+                    __stcs(a.L + (u64)bi.off + b[q] + (p - bi.soff) + 1, c);
                 }
                 if (st) last = p;
                 if (CODED && eq) depth = min(depth, D);
@@ -968,7 +968,7 @@ __global__ void __launch_bounds__(TPB) k_seg_emit1(FwdArgs a) {
             for (int q = 0; q < QB; q++) {
                 if (!((live >> q) & 1)) continue;
                 bv[q] = ch.blo == ch.bhi ? ch.blo : blk_of_pos(a, pv[q], ch.blo, ch.bhi);
-                idv[q] = pv[q] != gfv[q] ? (lsd_coded(a) ? (u32)__ldg(v.dep + pv[q]) : 0u) : ids ? __ldg(v.val + pv[q]) : 0u;
+                idv[q] = pv[q] != gfv[q] ? (lsd_coded(a) ? (u32)__ldg(v.dep + pv[q]) : 0u) : ids ? __ldcs(v.val + pv[q]) : 0u;
             }
 #pragma unroll
             for (int q = 0; q < QB; q++) {
@@ -1057,7 +1057,7 @@ __global__ void __launch_bounds__(TPB) k_seg_emit2(FwdArgs a) {
 #pragma unroll
             for (int q = 0; q < QB; q++) {
                 if (!((live >> q) & 1)) continue;
-                idv[q] = __ldg(v.val + pv[q]);
+                idv[q] = __ldcs(v.val + pv[q]);
                 giv[q] = __ldg(v.gidx + gfv[q]);
                 gbv[q] = __ldg(v.gbase + gfv[q]);
             }
