@@ -246,7 +246,7 @@ def single_blocks(workload: str, rank: int, mib: int):
 
 # DRAM bytes per unit (suffix) measured by ncu (dram__bytes_read.sum + dram__bytes_write.sum) on the 16 MiB prose
 # case: profiles/traffic_group_thread_lsd_pass_prose16.md (tiny groups) and profiles/lsd_pass_prose16.md (the
-# round-0 radix pass, averaged over a 16-pass step). The 64 MiB launch's traffic is scaled by the suffixes it
+# round-0 radix pass, averaged over the 8 passes of coded keys). The 64 MiB launch's traffic is scaled by the suffixes it
 # processes.
 TRAFFIC_PER_SUFFIX = {"group_thread": 35.1, "lsd_pass": 15.0}
 RANK_SORTERS = ("tile_sort_rank", "tile_warp_rank", "group_thread", "group_warp", "keygen")

@@ -6,8 +6,8 @@ tuning_gb300.json beside this package). Results never depend on the configuratio
 
 Tuned per bucket: CTAs per SM of the block tile kernel (tile_ctas) and of the bucket passes (msd_ctas), the
 counting-sort threshold of the tile kernel (small_group), the warp-level tile path (warp_path), the round-0 path
-(lsd_round0: one LSD radix sort of all suffixes, or bucket passes + tiles), the prefix it sorts (lsd_bytes: 16,
-which spares the first rank round, 12 or 8) and whether rank rounds follow repeat chains (chain_from: 1 or 0). The
+(lsd_round0: one LSD radix sort of all suffixes, or bucket passes + tiles), the key it sorts (lsd_bytes: 16 or
+12 bytes of text, or 8 of an order-preserving code of it) and whether rank rounds follow repeat chains (chain_from: 1 or 0). The
 tile capacity changes the workspace layout and is left at its default.
 """
 from __future__ import annotations

@@ -2,12 +2,15 @@
 //
 // Algorithm (Manber-Myers prefix doubling, as restated for GPUs by the reference's Metal sorter,
 // src/arch/metal/sa_metal.m:1-13 and src/arch/metal/sa.metal:178-256 of adnaneben/kolmo):
-//   round 0   group all suffixes by their first 8 bytes (zero padded past the block end);
-//   round j   h = 8 * 2^(j-1) characters are sorted; every suffix i still in a group of two or more ("active") is
-//             re-sorted inside its group by rank(i + h), where past the end of the block the key is below every
-//             rank and decreases with i (a shorter suffix sorts first: the reference's implicit sentinel);
+//   round 0   group all suffixes by their first characters (fwd_lsd.cuh: as many as 64 bits of an order-preserving
+//             code of the block's bytes hold whole, or 8, 12 or 16 bytes, zero padded past the block end);
+//   round j   h characters are sorted; every suffix i still in a group of two or more ("active") is re-sorted inside
+//             its group by rank(i + h), where past the end of the block the key is below every rank and decreases with
+//             i (a shorter suffix sorts first: the reference's implicit sentinel). In the round after a coded round 0
+//             each group uses the h of its own key, later ones twice the least of the round before;
 //   a suffix alone in its group is final: its rank is its suffix-array position.
-// The rank of a group is the suffix-array position of its first member (sa.metal:209-217).
+// The rank of a group is the suffix-array position of its first member (sa.metal:209-217), or, for large groups that
+// keep a label from an earlier round, of another position of its range, which orders the groups alike.
 //
 // GB300 formulation. There is no global sort per round. Groups are segments of an element list and are refined
 // in place of a sort:

@@ -50,7 +50,7 @@ struct Ctl {
     u64 cnt[NLISTS];  // per list: (segments << 32) | elements
     u32 rpar;         // round parity
     u32 pass;         // bucket pass within the round
-    u32 round;        // doubling round (0: 8-byte prefixes)
+    u32 round;        // doubling round (0: initial keys)
     u32 h;            // characters already sorted (rank rounds)
     u32 done;
     u32 err;
@@ -75,7 +75,7 @@ struct FwdConfig {
     int small_group = 64; // tiles whose groups are all at most this long skip the radix passes (counting sort)
     int warp_path = 1;    // tiles whose groups are all <= 32 long go to the warp-level kernel
     int lsd_round0 = 1;   // round 0 as one LSD radix sort of all suffixes; 0: bucket passes + tiles over 8-byte prefixes
-    int lsd_bytes = 16;   // bytes of the coded prefix the LSD round 0 sorts (8, 12 or 16)
+    int lsd_bytes = 16;   // bytes of the key the LSD round 0 sorts: 16 or 12 of text, or 8 of coded text
     int chain_from = 1;   // first rank round whose tiny groups may be ordered along their repeat chains (0: never)
 };
 // Fields of FwdConfig a caller set explicitly (they override the tuning table).
