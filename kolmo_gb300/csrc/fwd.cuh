@@ -65,7 +65,7 @@ struct Ctl {
     u32 p_alloc;        // slots taken so far in the tiny-group id array (shared by both parities, never reused)
     u32 idn;            // suffix ids of the batch lie in [0, idn) (the rank buffers' used extent)
     u32 prev_active;    // active suffixes of the round that just ended (the round-end kernel's last count)
-    u32 chain_go;       // this round follows repeat chains (doubling split less than a fifth of the actives)
+    u32 chain_go;       // this round follows repeat chains (doubling has stalled, most actives are in tiny groups)
 };
 
 struct FwdConfig {
