@@ -109,29 +109,56 @@ __device__ __forceinline__ u32 chunk_block(const InvArgs &a, u64 q) {
     return lo;
 }
 
-// Per-chunk byte histograms (a chunk is chunkt consecutive tiles of one block).
+// Per-chunk byte histograms (a chunk is chunkt consecutive tiles of one block), one per warp while counting. Bound by
+// the latency of its loads, so a thread has two 16-byte words in flight (byte loads, one in flight: 0.136 ms for 64 MiB
+// of prose and 0.39 for 216 MB of mixed blocks; now 0.042 and 0.155). BWT strings are full of short runs: a thread
+// counts each run inside its word with one atomic, which also keeps lanes off each other's counters.
 __global__ void __launch_bounds__(ITPB) k_inv_chunkhist(InvArgs a) {
-    __shared__ u32 h[256];
-    const u32 lane = lane_id();
+    constexpr int NW = ITPB / 32, HU = 2;  // 16-byte words a thread has in flight
+    __shared__ u32 h[NW][256];
+    const u32 t = threadIdx.x;
+    u32 *hw = h[warp_id()];
     for (u64 q = blockIdx.x; q < a.nchunk_all; q += gridDim.x) {
         const InvBlock B = a.blk[chunk_block(a, q)];
         const u32 start = (u32)(q - B.chunk_base) * (ITILE * a.chunkt);
         const u32 cnt = min(ITILE * a.chunkt, B.n - start);
         const u8 *src = a.U + (u64)B.off + start;
-        h[threadIdx.x] = 0;
+        // bytes before the first and after the last aligned word go one by one
+        const u32 head = min(cnt, (u32)(0 - (uintptr_t)src) & 15u), nv = (cnt - head) / 16, tail = (cnt - head) & 15u;
+        const uint4 *words = reinterpret_cast<const uint4 *>(src + head);
+#pragma unroll
+        for (int w = 0; w < NW; w++) h[w][t] = 0;
         __syncthreads();
-        for (u32 i0 = 0; i0 < cnt; i0 += ITPB) {
-            const u32 i = i0 + threadIdx.x;
-            const u32 c = i < cnt ? (u32)src[i] : 0x100u;
-            // (runs of one byte would serialise 32 atomics on one counter)
-            if (__all_sync(0xffffffffu, c == __shfl_sync(0xffffffffu, c, 0))) {
-                if (c < 256 && lane == 0) atomicAdd(&h[c], 32u);
-            } else if (c < 256) {
-                atomicAdd(&h[c], 1u);
+        if (t < head) atomicAdd(&hw[src[t]], 1u);
+        if (t < tail) atomicAdd(&hw[src[head + nv * 16 + t]], 1u);
+        for (u32 i0 = t; i0 < nv; i0 += HU * ITPB) {
+            uint4 v[HU];
+#pragma unroll
+            for (int k = 0; k < HU; k++)
+                if (i0 + k * ITPB < nv) v[k] = __ldg(words + i0 + k * ITPB);
+#pragma unroll
+            for (int k = 0; k < HU; k++) {
+                if (i0 + k * ITPB >= nv) break;
+                const u32 w[4] = {v[k].x, v[k].y, v[k].z, v[k].w};
+                u32 cur = w[0] & 255u, len = 1;  // the run in progress
+#pragma unroll
+                for (int p = 1; p < 16; p++) {
+                    const u32 c = __byte_perm(w[p / 4], 0, 0x4440 + p % 4);
+                    if (c != cur) {
+                        atomicAdd(&hw[cur], len);
+                        cur = c;
+                        len = 0;
+                    }
+                    len++;
+                }
+                atomicAdd(&hw[cur], len);
             }
         }
         __syncthreads();
-        a.csum[q * 256 + threadIdx.x] = h[threadIdx.x];
+        u32 sum = 0;
+#pragma unroll
+        for (int w = 0; w < NW; w++) sum += h[w][t];
+        a.csum[q * 256 + t] = sum;
         __syncthreads();
     }
 }
