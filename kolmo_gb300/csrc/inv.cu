@@ -23,11 +23,15 @@
 // That block is reported (-1) instead of decoded. Every loop is bounded by the number of rows.
 #include "inv.cuh"
 
+#include <cooperative_groups.h>
+
 #include <algorithm>
 #include <cstring>
 #include <mutex>
 
 #include "kgbwt.h"
+
+namespace cg = cooperative_groups;
 
 namespace kgb {
 
@@ -47,7 +51,11 @@ constexpr u32 FT_LOG = 10, FT = 1u << FT_LOG;
 // Tiles per chunk of the psi build: 16 on large batches, halved while the batch has at most CHUNKS_MIN chunks, so that
 // small ones fill the GPU (a 1 MiB block: 256 chunks of one tile instead of 16 of 16).
 constexpr u32 CHUNKT = 16, CHUNKS_MIN = 1024;
-constexpr int STPB = 1024;   // threads of the chunk scan: four per byte value
+constexpr int STPB = 1024;   // threads of the chunk scan
+// Its CTAs per block where blocks average more than so many chunks and the clusters fit the GPU at once. One block of 5,
+// 32, 256 or 1024 chunks: 7, 8, 14 or 38 us with one CTA and 8, 9, 9.5 or 12.5 with eight; 64 blocks of 16 or 32 chunks: 8
+// and 24, 400 blocks: 12.5 and 108.
+constexpr u32 SCL = 8, SCL_CHUNKS = 64;
 
 struct InvArgs {
     const u8 *U;
@@ -163,67 +171,92 @@ __global__ void __launch_bounds__(ITPB) k_inv_chunkhist(InvArgs a) {
     }
 }
 
-// Per block: C array (C[c] = 1 + number of bytes below c: F row 0 is the sentinel) and the exclusive scan of the
-// chunk histograms, so csum[q][c] becomes the first psi slot of chunk q's c bytes.
-// Four threads share a byte value, each a quarter of the chunks (eight loads in flight).
-__global__ void __launch_bounds__(STPB) k_inv_chunkscan(InvArgs a) {
+// Per block: C array (C[c] = 1 + number of bytes below c: F row 0 is the sentinel), the table from a row's leading bits
+// to its byte values, and the exclusive scan of the chunk histograms, so csum[q][c] becomes the first psi slot of chunk
+// q's c bytes. CL CTAs share a block, each a slice of the byte values, whose totals they read from each other's shared
+// memory; the threads of a CTA that share a byte value take consecutive chunks. One CTA is bound by what one SM reads
+// and writes (1 MB of counts three times for a 64 MiB block).
+template <int CL>
+__device__ __forceinline__ void chunk_scan(const InvArgs &a) {
+    constexpr u32 CW = 256 / CL, G = STPB / CW;
     __shared__ u32 ws[STPB / 32 + 1];
-    __shared__ u32 part[4][256];
+    __shared__ u32 part[G][CW];
+    __shared__ u32 tots[CW];
     __shared__ u32 first[257];
-    const u32 c = threadIdx.x & 255, g = threadIdx.x >> 8;
-    for (u32 b = blockIdx.x; b < a.B; b += gridDim.x) {
+    const u32 t = threadIdx.x, k = t % CW, g = t / CW, rank = CL > 1 ? blockIdx.x % CL : 0;
+    const u32 c = rank * CW + k;
+    for (u32 b = blockIdx.x / CL; b < a.B; b += gridDim.x / CL) {  // (the same blocks for every CTA of a cluster)
         const InvBlock B = a.blk[b];
         u32 *col = a.csum + (u64)B.chunk_base * 256 + c;
-        const u32 per = (B.nchunk + 3) / 4, q0 = min(B.nchunk, g * per), q1 = min(B.nchunk, q0 + per);
+        const u32 per = (B.nchunk + G - 1) / G, q0 = min(B.nchunk, g * per), q1 = min(B.nchunk, q0 + per);
         u32 tot = 0;
         u32 q = q0;
         for (; q + 8 <= q1; q += 8) {
             u32 v[8];
 #pragma unroll
-            for (int k = 0; k < 8; k++) v[k] = col[(u64)(q + k) * 256];
+            for (int i = 0; i < 8; i++) v[i] = col[(u64)(q + i) * 256];
 #pragma unroll
-            for (int k = 0; k < 8; k++) tot += v[k];
+            for (int i = 0; i < 8; i++) tot += v[i];
         }
         for (; q < q1; q++) tot += col[(u64)q * 256];
-        part[g][c] = tot;
+        part[g][k] = tot;
         __syncthreads();
+        if (g == 0) {
+            u32 sum = 0;
+            for (u32 w = 0; w < G; w++) sum += part[w][k];
+            tots[k] = sum;
+        }
         u32 sum = 0;
-        if (g == 0) sum = part[0][c] + part[1][c] + part[2][c] + part[3][c];
+        if constexpr (CL > 1) {
+            cg::cluster_group cl = cg::this_cluster();
+            cl.sync();
+            if (t < 256) sum = *cl.map_shared_rank(&tots[t % CW], t / CW);
+        } else {
+            __syncthreads();
+            if (t < 256) sum = tots[t];
+        }
         u32 all;
         const u32 cc = 1 + block_excl_sum<STPB>(sum, ws, &all);  // (threads 0..255 carry the sums)
-        if (g == 0) {
-            first[c] = cc;
-            a.C[(u64)b * 257 + c] = cc;
-            if (c == 255) a.C[(u64)b * 257 + 256] = first[256] = 1 + all;
+        if (t < 256) {
+            first[t] = cc;
+            if (t / CW == rank) a.C[(u64)b * 257 + t] = cc;
+            if (t == 255) {
+                first[256] = 1 + all;
+                if (rank == CL - 1) a.C[(u64)b * 257 + 256] = 1 + all;
+            }
         }
         __syncthreads();
-        {
+        static_assert(FT == STPB, "one entry per thread");
+        if (t < FT / CL) {
+            const u32 e = rank * (FT / CL) + t;
             const u32 sh = ft_shift(B.n);
-            static_assert(FT == STPB, "one entry per thread");
-            const u64 r0 = (u64)threadIdx.x << sh, r1 = ((u64)(threadIdx.x + 1) << sh) - 1;
+            const u64 r0 = (u64)e << sh, r1 = ((u64)(e + 1) << sh) - 1;
             const u32 lo = f_search(first, (u32)max(r0, (u64)1), 0, 255);
             const u32 hi = f_search(first, (u32)min(r1, (u64)B.n), 0, 255);
-            a.ft[(u64)b * FT + threadIdx.x] = (u16)(lo | max(lo, hi) << 8);
+            a.ft[(u64)b * FT + e] = (u16)(lo | max(lo, hi) << 8);
         }
         u32 run = first[c];
-        for (u32 w = 0; w < g; w++) run += part[w][c];
+        for (u32 w = 0; w < g; w++) run += part[w][k];
         q = q0;
         for (; q + 8 <= q1; q += 8) {
             u32 v[8];
 #pragma unroll
-            for (int k = 0; k < 8; k++) v[k] = col[(u64)(q + k) * 256];
+            for (int i = 0; i < 8; i++) v[i] = col[(u64)(q + i) * 256];
 #pragma unroll
-            for (int k = 0; k < 8; k++) { col[(u64)(q + k) * 256] = run; run += v[k]; }
+            for (int i = 0; i < 8; i++) { col[(u64)(q + i) * 256] = run; run += v[i]; }
         }
         for (; q < q1; q++) {
             const u32 v = col[(u64)q * 256];
             col[(u64)q * 256] = run;
             run += v;
         }
-        if (threadIdx.x == 0) a.psi[(u64)B.off + b] = B.p0 | 0x80000000u;  // psi[0]: the sentinel row leads to row p0
-        __syncthreads();  // part and first are free for the next block
+        if (t == 0 && rank == 0) a.psi[(u64)B.off + b] = B.p0 | 0x80000000u;  // psi[0]: the sentinel row leads to row p0
+        if constexpr (CL > 1) cg::this_cluster().sync();  // the others have read tots: free for the next block, or to exit
+        else __syncthreads();
     }
 }
+__global__ void __launch_bounds__(STPB) k_inv_chunkscan(InvArgs a) { chunk_scan<1>(a); }
+__global__ void __cluster_dims__(SCL, 1, 1) __launch_bounds__(STPB) k_inv_chunkscan_cl(InvArgs a) { chunk_scan<SCL>(a); }
 
 // Stable scatter, one CTA per chunk walking its tiles in order: psi[C[c] + occurrences of c before row q] = q,
 // with the mark flag of q.
@@ -675,7 +708,11 @@ int InvEngine::enqueue(cudaStream_t s, long long *launches) {
     const u32 nbytes = (u32)std::min<u64>(N, 0xFFFFFFFFull);
     const int gch = (int)std::min<u64>(nchunk_all, (u64)sm_count * 8);
     KGB_CHECK(go(K_INV_TILEHIST, nbytes, [&] { k_inv_chunkhist<<<gch, ITPB, 0, s>>>(a); }));
-    KGB_CHECK(go(K_INV_COLSCAN, (u32)nchunk_all, [&] { k_inv_chunkscan<<<(int)std::min<u32>(B, 4096u), STPB, 0, s>>>(a); }));
+    KGB_CHECK(go(K_INV_COLSCAN, (u32)nchunk_all, [&] {
+        const u32 nb = std::min<u32>(B, 4096u);
+        if (nchunk_all > (u64)B * SCL_CHUNKS && B * SCL <= (u32)sm_count) k_inv_chunkscan_cl<<<nb * SCL, STPB, 0, s>>>(a);
+        else k_inv_chunkscan<<<nb, STPB, 0, s>>>(a);
+    }));
     KGB_CHECK(go(K_INV_SCATTER, nbytes, [&] { k_inv_scatter<<<gch, ITPB, 0, s>>>(a); }));
     // the CTAs the GPU holds at once, or fewer when there are fewer chains than threads
     const int gw = (int)std::max<u64>(1, std::min<u64>((u64)walk_grid, ((u64)nwalk + ITPB - 1) / ITPB));
