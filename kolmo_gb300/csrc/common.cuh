@@ -76,8 +76,8 @@ __device__ __forceinline__ u32 warp_sum(u32 v) {
 // ballot each) and, for the rest, by collecting lane bits with one shared-memory atomic. __match_any_sync takes two
 // cycles per SM and distinct digit: 59 for 32 lanes of evenly spread digits, 27 for letters of text, 5 for four
 // values; the atomics alone take 10, 11 and 14, but 36 where one digit fills the warp; with the pivots it is 12, 12 and
-// 14, and 8 there. Q elements in flight hide the atomics' latency; one lane per digit advances the counter for all
-// (atomics of one warp to shared memory take effect in program order).
+// 14, and 8 there. Q elements in flight hide the mask atomics' latency; one lane per digit advances the counter for all,
+// and as that lane differs from element to element, a warp barrier puts the elements' counts in order.
 template <int Q, bool CHECK>
 __device__ __forceinline__ void warp_rank(u32 *mask, u32 *cnt, const u32 (&d)[Q], u32 (&rank)[Q]) {
     const u32 all = 0xffffffffu, bit = 1u << lane_id();
@@ -105,6 +105,7 @@ __device__ __forceinline__ void warp_rank(u32 *mask, u32 *cnt, const u32 (&d)[Q]
             rank[q] = atomicAdd(cnt + d[q], (u32)__popc(peers[q]));
             if (rest[q]) mask[256 * q + d[q]] = 0;
         }
+        __syncwarp();  // element q's counts before element q + 1's, which other lanes add
     }
 #pragma unroll
     for (int q = 0; q < Q; q++)
