@@ -130,7 +130,8 @@ int32_t kgbwt_engine_last_config_n(kgbwt_engine *e, int32_t *cfg, int32_t ncfg);
  * iout (dI[iout] = primary index), dSA (may be NULL) the suffix array at off. */
 int32_t kgbwt_engine_fwd(kgbwt_engine *e, const uint8_t *dT, uint8_t *dL, int32_t *dI, int32_t *dSA,
                          const kgbwt_block *blocks, int32_t count, void *stream, uint32_t flags);
-/* Inverse: BWT strings (sentinel removed, as the drop-in U) in dU; decoded texts into dOut at the same offsets. */
+/* Inverse: BWT strings (sentinel removed, as the drop-in U) in dU; decoded texts into dOut at the same offsets. Blocks
+ * may be listed in any order. */
 int32_t kgbwt_engine_inv(kgbwt_engine *e, const uint8_t *dU, uint8_t *dOut, const kgbwt_iblock *blocks,
                          int32_t count, void *stream, uint32_t flags);
 /* Waits for the engine's last enqueued call. status (may be NULL) receives one code per block of an inverse call

@@ -250,7 +250,7 @@ __device__ __forceinline__ void chunk_scan(const InvArgs &a) {
             col[(u64)q * 256] = run;
             run += v;
         }
-        if (t == 0 && rank == 0) a.psi[(u64)B.off + b] = B.p0 | 0x80000000u;  // psi[0]: the sentinel row leads to row p0
+        if (t == 0 && rank == 0) a.psi[B.psi_base] = B.p0 | 0x80000000u;  // psi[0]: the sentinel row leads to row p0
         if constexpr (CL > 1) cg::this_cluster().sync();  // the others have read tots: free for the next block, or to exit
         else __syncthreads();
     }
@@ -275,7 +275,7 @@ __global__ void __launch_bounds__(ITPB, 3) k_inv_scatter(InvArgs a) {
         const u32 cstart = (u32)(q - B.chunk_base) * (ITILE * a.chunkt);
         const u32 ccnt = min(ITILE * a.chunkt, B.n - cstart);
         run_s[threadIdx.x] = a.csum[q * 256 + threadIdx.x];
-        u32 *psi = a.psi + (u64)B.off + b;
+        u32 *psi = a.psi + B.psi_base;
         for (u32 t0 = 0; t0 < ccnt; t0 += ITILE) {
             const u32 start = cstart + t0;
             const u32 cnt = min(ITILE, ccnt - t0);
@@ -377,7 +377,7 @@ __global__ void __launch_bounds__(ITPB, 6) k_inv_walk(InvArgs a) {
             const InvBlock B = a.blk[b];
             const u32 id = q - B.qbase, start = chain_start(id, B);
             if (start == 0) continue;  // no such row, or chain 0 covers the mark at p0
-            psi = a.psi + (u64)B.off + b;
+            psi = a.psi + B.psi_base;
             bn = B.n;
             sh = ft_shift(B.n);
             row = start; steps = 0; rec = B.chain_base + id;
@@ -524,15 +524,16 @@ void InvEngine::free_all() {
     pool = nullptr;
     if (h_status) cudaFreeHost(h_status);
     h_status = nullptr;
-    Ncap = Tcap = Ccap = 0; Bcap = 0;
+    Ncap = Tcap = Ccap = Pcap = 0; Bcap = 0;
 }
 
-// The workspace for ncap text bytes, bcap blocks, tcap psi-build chunks and ccap chain records, in pool order.
+// The workspace for ncap text bytes, bcap blocks, tcap psi-build chunks, ccap chain records and pcap psi rows, in pool
+// order.
 template <typename Add>
-void InvEngine::layout(u64 ncap, u32 bcap, u64 tcap, u64 ccap, Add add) {
+void InvEngine::layout(u64 ncap, u32 bcap, u64 tcap, u64 ccap, u64 pcap, Add add) {
     add((void **)&own_U, ncap + 64);
     add((void **)&own_out, ncap + 64);
-    add((void **)&d_psi, (ncap + bcap + 16) * 4);
+    add((void **)&d_psi, (pcap + 16) * 4);
     add((void **)&d_csum, tcap * 256 * 4);
     add((void **)&d_C, (size_t)bcap * 257 * 4);
     add((void **)&d_ft, (size_t)bcap * FT * 2);
@@ -544,15 +545,16 @@ void InvEngine::layout(u64 ncap, u32 bcap, u64 tcap, u64 ccap, Add add) {
     add((void **)&d_status, (size_t)bcap * 4);
 }
 
-int InvEngine::grow(u64 ncap, u32 bcap, u64 tcap, u64 ccap) {
-    if (ncap <= Ncap && bcap <= Bcap && tcap <= Tcap && ccap <= Ccap) return 0;
+int InvEngine::grow(u64 ncap, u32 bcap, u64 tcap, u64 ccap, u64 pcap) {
+    if (ncap <= Ncap && bcap <= Bcap && tcap <= Tcap && ccap <= Ccap && pcap <= Pcap) return 0;
     ncap = std::max(ncap, Ncap); bcap = std::max(bcap, Bcap); tcap = std::max(tcap, Tcap); ccap = std::max(ccap, Ccap);
+    pcap = std::max(pcap, Pcap);
     if (gexec) { cudaGraphExecDestroy(gexec); gexec = nullptr; }
     if (graph) { cudaGraphDestroy(graph); graph = nullptr; }
     if (pool) { cudaFree(pool); pool = nullptr; }
     struct Item { void **p; size_t bytes; };
     std::vector<Item> items;
-    layout(ncap, bcap, tcap, ccap,
+    layout(ncap, bcap, tcap, ccap, pcap,
            [&](void **p, size_t bytes) { items.push_back({p, ialign(std::max<size_t>(bytes, 16), 256)}); });
     size_t total = 0;
     for (auto &it : items) total += it.bytes;
@@ -568,7 +570,7 @@ int InvEngine::grow(u64 ncap, u32 bcap, u64 tcap, u64 ccap) {
     for (auto &it : items) { *it.p = (char *)pool + off; off += it.bytes; }
     if (h_status) cudaFreeHost(h_status);
     KGB_CHECK(cudaMallocHost(&h_status, (size_t)bcap * sizeof(int)));
-    Ncap = ncap; Bcap = bcap; Tcap = tcap; Ccap = ccap;
+    Ncap = ncap; Bcap = bcap; Tcap = tcap; Ccap = ccap; Pcap = pcap;
     return 0;
 }
 
@@ -592,9 +594,10 @@ static u32 mark_of(const u32 *n, int count) {
 
 static int plan_layout(const u32 *off, const u32 *n, const u32 *p0, int count, std::vector<InvBlock> &blk,
                        u64 &nchunk_all, u64 &nchains, u32 &chunkt,
-                       u32 &nwalk) {
+                       u32 &nwalk, u64 &nrows) {
     blk.resize(count);
     nwalk = 0;
+    nrows = 0;
     const u32 mark = mark_of(n, count);
     nchunk_all = 0; nchains = 0;
     auto chunks_of = [&](u32 t) {
@@ -614,6 +617,8 @@ static int plan_layout(const u32 *off, const u32 *n, const u32 *p0, int count, s
         B.chain_base = (u32)nchains;
         B.chain_cap = B.nreg + 1 + n[b] / CAPC + 4;
         B.qbase = nwalk;
+        B.psi_base = nrows;
+        nrows += (u64)n[b] + 1;
         nwalk += B.nreg + 1;
         nchunk_all += B.nchunk;
         nchains += B.chain_cap;
@@ -628,12 +633,12 @@ u64 InvEngine::estimate_bytes(const u32 *n, int count) {
     u64 o = 0;
     for (int b = 0; b < count; b++) { off[b] = (u32)o; o += ((u64)n[b] + 15) / 16 * 16; }
     std::vector<InvBlock> blk;
-    u64 nch = 0, nchains_ = 0;
+    u64 nch = 0, nchains_ = 0, nr = 0;
     u32 ct = 0, nw = 0;
-    if (plan_layout(off.data(), n, p0.data(), count, blk, nch, nchains_, ct, nw)) return ~0ull;
+    if (plan_layout(off.data(), n, p0.data(), count, blk, nch, nchains_, ct, nw, nr)) return ~0ull;
     u64 total = 0;
     layout(std::max<u64>(o, Ncap), std::max<u32>((u32)count, Bcap), std::max<u64>(nch, Tcap),
-           std::max<u64>(nchains_, Ccap),
+           std::max<u64>(nchains_, Ccap), std::max<u64>(nr, Pcap),
            [&](void **, size_t bytes) { total += ialign(std::max<size_t>(bytes, 16), 256); });
     return total;
 }
@@ -656,9 +661,9 @@ int InvEngine::plan(const u32 *n, const u32 *p0, int count) {
         off += ((u64)n[b] + 15) / 16 * 16;
         if (off > 0xFFFF0000ull) return -1;
     }
-    if (plan_layout(h_off.data(), n, p0, count, h_blk, nchunk_all, nchains, chunkt, nwalk)) return -1;
+    if (plan_layout(h_off.data(), n, p0, count, h_blk, nchunk_all, nchains, chunkt, nwalk, nrows)) return -1;
     N = off; B = (u32)count;
-    int rc = grow(N, B, nchunk_all, nchains);
+    int rc = grow(N, B, nchunk_all, nchains, nrows);
     if (rc) return rc;
     ext = false;
     d_U = own_U; d_out = own_out;
@@ -669,11 +674,11 @@ int InvEngine::plan_external(const u32 *off, const u32 *n, const u32 *p0, int co
     if (count <= 0) return -1;
     if (int rc = uploads_done()) return rc;
     h_off.assign(off, off + count);
-    if (plan_layout(off, n, p0, count, h_blk, nchunk_all, nchains, chunkt, nwalk)) return -1;
+    if (plan_layout(off, n, p0, count, h_blk, nchunk_all, nchains, chunkt, nwalk, nrows)) return -1;
     u64 end = 0;
     for (int b = 0; b < count; b++) end = std::max<u64>(end, (u64)off[b] + n[b]);
     N = end; B = (u32)count;
-    int rc = grow(N, B, nchunk_all, nchains);
+    int rc = grow(N, B, nchunk_all, nchains, nrows);
     if (rc) return rc;
     ext = true;
     d_U = dU; d_out = dOut;
@@ -831,7 +836,7 @@ static int unbwt_noalloc(const u8 *dU, u8 *dT, u32 n, u32 p0, cudaStream_t s) {
     InvBlock B;
     B.off = 0; B.n = n; B.p0 = p0;
     B.chunk_base = 0; B.nchunk = (n + ITILE - 1) / ITILE;
-    B.nreg = n / MARK; B.chain_base = 0; B.chain_cap = B.nreg + 1 + n / CAPC + 4; B.qbase = 0;
+    B.nreg = n / MARK; B.chain_base = 0; B.chain_cap = B.nreg + 1 + n / CAPC + 4; B.qbase = 0; B.psi_base = 0;
     mark_params(B);
     KGB_CHECK(cudaMemcpyAsync(S->blk, &B, sizeof(B), cudaMemcpyHostToDevice, s));
     // the array keeps the previous call's contents: reset what must start at zero (or at "no successor")

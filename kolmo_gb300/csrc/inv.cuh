@@ -19,6 +19,8 @@ struct InvBlock {
     u32 hmul;        // odd multiplier: the top k bits of 2^64 / golden ratio (rows of the marks are a Weyl sequence)
     u32 hinv;        // hmul^-1 mod 2^32: row q is mark (q * hinv) & hmask
     u32 qbase;       // the block's chains in the walk's sequence over all blocks: qbase .. qbase + nreg
+    u64 psi_base;    // first psi row of the block (rows 0..n): the tables follow each other in the order of the blocks
+                     // in the call, whatever their offsets
 };
 
 struct InvStats {
@@ -48,17 +50,17 @@ class InvEngine {
     u64 estimate_bytes(const u32 *n, int count);
 
    private:
-    int grow(u64 ncap, u32 bcap, u64 tcap, u64 ccap);
+    int grow(u64 ncap, u32 bcap, u64 tcap, u64 ccap, u64 pcap);
     template <typename Add>
-    void layout(u64 ncap, u32 bcap, u64 tcap, u64 ccap, Add add);
+    void layout(u64 ncap, u32 bcap, u64 tcap, u64 ccap, u64 pcap, Add add);
     int build_graph(cudaStream_t s);
     int enqueue(cudaStream_t s, long long *launches);
     u32 nmax() const;
     int uploads_done();
     void free_all();
-    u64 Ncap = 0, Tcap = 0, Ccap = 0;
+    u64 Ncap = 0, Tcap = 0, Ccap = 0, Pcap = 0;
     u32 Bcap = 0;
-    u64 N = 0, nchunk_all = 0, nchains = 0;
+    u64 N = 0, nchunk_all = 0, nchains = 0, nrows = 0;
     u32 B = 0, chunkt = 0, nwalk = 0;
     int walk_grid = 0;   // resident CTAs of the walk kernel
     std::vector<u32> h_off;
