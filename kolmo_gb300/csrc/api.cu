@@ -163,6 +163,13 @@ static uint32_t env_flags() {
     return plain ? KGBWT_PLAIN : 0u;
 }
 
+// Before a failed call returns: copies from or to the callers' buffers may be queued, and a caller is free to reuse its
+// buffers after the return. The first error is on record; what the wait adds to it is dropped.
+static void settle(cudaStream_t s) {
+    cudaStreamSynchronize(s);
+    cudaGetLastError();
+}
+
 int run_fwd_jobs(Worker &C, kgbwt_fwd_job *jobs, int32_t count, uint32_t flags) {
     std::vector<int> dev;
     std::vector<u32> n, r;
@@ -186,7 +193,7 @@ int run_fwd_jobs(Worker &C, kgbwt_fwd_job *jobs, int32_t count, uint32_t flags) 
     int rc = E.plan(n.data(), r.data(), (int)dev.size(), false);
     if (rc) { for (int i : dev) jobs[i].rc = rc; return rc; }
     cudaStream_t s = C.stream;
-    auto fail = [&](int code) { for (int i : dev) jobs[i].rc = code; return code; };
+    auto fail = [&](int code) { settle(s); for (int i : dev) jobs[i].rc = code; return code; };
     for (size_t k = 0; k < dev.size(); k++) {
         if (cudaMemcpyAsync(E.text() + E.offsets()[k], jobs[dev[k]].T, n[k], cudaMemcpyHostToDevice, s) != cudaSuccess)
             return fail(record_cuda_error(cudaGetLastError(), "cudaMemcpyAsync(text)", __FILE__, __LINE__));
@@ -232,11 +239,17 @@ int run_fwd_jobs(Worker &C, kgbwt_fwd_job *jobs, int32_t count, uint32_t flags) 
         return fail(-2);
     }
     const u32 *I = reinterpret_cast<const u32 *>(C.stage_I.p);
+    for (size_t k = 0; k < dev.size(); k++) {  // (before any buffer is written)
+        const u32 p0 = I[E.iouts()[k]];
+        if (p0 < 1 || p0 > n[k]) {
+            record_error("forward sort: primary index out of range (internal error)");
+            return fail(-2);
+        }
+    }
     const u8 *SL = C.stage_L.p;
     for (size_t k = 0; k < dev.size(); k++) {
         kgbwt_fwd_job &j = jobs[dev[k]];
         const u32 p0 = I[E.iouts()[k]];
-        if (p0 < 1 || p0 > (u32)j.n) return fail(-2);
         if (!direct[k]) {
             memcpy(j.U, SL, p0);
             memcpy(j.U + p0, SL + p0 + 1, (size_t)j.n - p0);
@@ -285,9 +298,9 @@ int run_inv_jobs(Worker &C, kgbwt_inv_job *jobs, int32_t count, uint32_t flags) 
     if (int rc = C.init()) { for (int i : dev) jobs[i].rc = rc; return rc; }
     InvEngine &E = C.eng.inv;
     int rc = E.plan(n.data(), p0.data(), (int)dev.size());
-    auto fail = [&](int code) { for (int i : dev) jobs[i].rc = code; return code; };
-    if (rc) return fail(rc);
+    if (rc) { for (int i : dev) jobs[i].rc = rc; return rc; }
     cudaStream_t s = C.stream;
+    auto fail = [&](int code) { settle(s); for (int i : dev) jobs[i].rc = code; return code; };
     for (size_t k = 0; k < dev.size(); k++)
         if (cudaMemcpyAsync(E.input() + E.offsets()[k], jobs[dev[k]].T, n[k], cudaMemcpyHostToDevice, s) != cudaSuccess)
             return fail(record_cuda_error(cudaGetLastError(), "cudaMemcpyAsync(bwt)", __FILE__, __LINE__));
