@@ -1776,7 +1776,7 @@ __global__ void k_ctl_msd_next(FwdArgs a) {
     if (p == 0) c->cnt[L_L0 + c->rpar] = 0; else c->cnt[L_K0 + ((p - 1) & 1)] = 0;
     c->pass = p + 1;
     const u32 more = elems(c, produced) > 0;
-    if (p + 1 > 2 * DEPTH_PREFIX + 2) { c->err |= 2; set_cond(a.hcond, 0); return; }
+    if (p + 1 > 2 * DEPTH_PREFIX + 2) { atomicOr(&c->err, 2u); set_cond(a.hcond, 0); return; }  // (other kernels run beside)
     set_cond(a.hcond, more);
 }
 __global__ void k_ctl_round_end(FwdArgs a) {
@@ -1805,7 +1805,7 @@ __global__ void k_ctl_round_end(FwdArgs a) {
     c->prev_active = active;
     c->pass = 0;
     u32 cont = active > 0;
-    if (cont && c->round > c->maxrounds) { c->err |= 1; cont = 0; }
+    if (cont && c->round > c->maxrounds) { atomicOr(&c->err, 1u); cont = 0; }
     c->done = !cont;
     set_cond(a.hcond, cont);
 }
