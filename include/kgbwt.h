@@ -127,7 +127,9 @@ int32_t kgbwt_tuning_lookup_n(uint64_t n, int32_t *cfg, int32_t ncfg);
 int32_t kgbwt_engine_last_config_n(kgbwt_engine *e, int32_t *cfg, int32_t ncfg);
 /* Forward: text blocks in dT (16 readable bytes past the last block). Results: dL receives each block's L column
  * with its sentinel row (n + 1 bytes at off + block index; row p0 holds no text byte), dI the sampled indexes at
- * iout (dI[iout] = primary index), dSA (may be NULL) the suffix array at off. */
+ * iout (dI[iout] = primary index), dSA (may be NULL) the suffix array at off. dT is 8-byte aligned. Blocks must not
+ * overlap (-1). The L columns of blocks listed by ascending offset never share a byte of dL; in another order they do not
+ * where at least `count` bytes lie between any two blocks. */
 int32_t kgbwt_engine_fwd(kgbwt_engine *e, const uint8_t *dT, uint8_t *dL, int32_t *dI, int32_t *dSA,
                          const kgbwt_block *blocks, int32_t count, void *stream, uint32_t flags);
 /* Inverse: BWT strings (sentinel removed, as the drop-in U) in dU; decoded texts into dOut at the same offsets. Blocks

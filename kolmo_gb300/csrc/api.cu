@@ -690,6 +690,20 @@ int32_t kgbwt_engine_option(kgbwt_engine *e, int32_t option, int32_t value) {
     }
 }
 
+// Whether two blocks of the list share a byte (any order).
+static bool overlapping(const std::vector<u32> &off, const std::vector<u32> &n) {
+    const size_t count = off.size();
+    bool ascending = true;
+    for (size_t b = 1; b < count && ascending; b++) ascending = (u64)off[b - 1] + n[b - 1] <= off[b];
+    if (ascending) return false;
+    std::vector<u32> at(count);
+    for (size_t b = 0; b < count; b++) at[b] = (u32)b;
+    std::sort(at.begin(), at.end(), [&](u32 x, u32 y) { return off[x] < off[y]; });
+    for (size_t b = 1; b < count; b++)
+        if ((u64)off[at[b - 1]] + n[at[b - 1]] > off[at[b]]) return true;
+    return false;
+}
+
 int32_t kgbwt_engine_fwd(kgbwt_engine *e, const uint8_t *dT, uint8_t *dL, int32_t *dI, int32_t *dSA,
                          const kgbwt_block *blocks, int32_t count, void *stream, uint32_t flags) {
     if (!e || !dT || !dL || !dI || !blocks || count <= 0) return -1;
@@ -700,6 +714,8 @@ int32_t kgbwt_engine_fwd(kgbwt_engine *e, const uint8_t *dT, uint8_t *dL, int32_
         if (blocks[b].n < 2 || bad_r((int32_t)blocks[b].r) || blocks[b].n > 0x7FFFFFFFu) return -1;
         off[b] = blocks[b].off; n[b] = blocks[b].n; r[b] = blocks[b].r; io[b] = blocks[b].iout;
     }
+    // (the workspace has one element per byte of the batch's extent, and ranks are kept per text position)
+    if (overlapping(off, n)) { record_error("the blocks of a forward call must not overlap"); return -1; }
     if (int rc = refuse_capture((cudaStream_t)stream)) return rc;
     int rc = e->fwd.plan_external(off.data(), n.data(), r.data(), io.data(), count, const_cast<uint8_t *>(dT), dL,
                                   reinterpret_cast<u32 *>(dI), reinterpret_cast<u32 *>(dSA));
