@@ -34,9 +34,12 @@ constexpr u64 ST_EPOCH = 0xFFFFFFFF00000000ull;
 constexpr int LB_WIN = 4;  // look-back window (predecessor words read per step; 8: 0.5% slower on 64 MiB of prose)
 
 // Which keys: the tuning table's choice per batch size, by measurement; it takes coded keys throughout. They halve the
-// passes, compare more in the segmentation and leave slightly larger groups. Forward call, coded against raw 16 bytes:
-// log lines 20 KB 0.20 ms against 0.22, 1 MiB 0.41 and 0.44, 30 MB 5.65 and 5.95; prose 1 MiB 0.49 and 0.55, 64 slices of
-// 512 KiB 4.18 and 5.34, 64 MiB 14.48 and 14.70; 48 MiB Markov 5.39 and 7.90; 16 mixed blocks (53 MB) 8.00 and 11.17.
+// passes, compare more in the segmentation and leave slightly larger groups. Forward call in ms at 1, 4, 16 and 64 MiB,
+// coded against raw 16 bytes (medians of 7 rounds in turn, which agree within 1%): log lines 0.39 0.87 2.98 12.63 against
+// 0.45 1.00 3.27 12.98, Markov bytes 0.22 0.51 1.65 7.50 against 0.36 0.92 2.76 10.72, prose 0.48 0.98 3.48 14.81 against
+// 0.47 1.17 3.80 14.74, prose copied over and over 1.40 3.45 6.19 (to 16 MiB) against 1.37 3.50 6.24; 96 mixed blocks 36.5
+// against 41.0. So prose gains in the middle sizes only and is 2% slower at 1 MiB (0.5% at 64), which a rule by size
+// cannot tell from the texts that gain 3-38% there.
 // Raw keys stay for engines that ask for 12 or 16 bytes and where no table is loaded.
 __host__ __device__ __forceinline__ bool lsd_coded(const FwdArgs &a) { return a.lsd_bytes == 8; }
 __device__ __forceinline__ u32 active_slots(const Ctl *c) { return c->lsd_act; }  // bit s: slot s varies
