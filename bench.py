@@ -21,8 +21,8 @@ Output: one JSON line on rank 0.
   cpu_baseline  the reference's own CPU sorter (compiled on this host from the reference's sources by
           oracle/Makefile) on the whole workload with all host threads, and with one ("t1"); where it is not
           available, the CPU restatement in oracle/ on a bounded sample.
---impl reference times the reference's own CPU sorter (else the restatement) on the same workload, each step the
-whole workload, with all host threads.
+--impl reference times the reference's own CPU sorter on the same workload, each step the whole workload, with all host
+threads; where that sorter is not built its line says "unavailable".
 """
 from __future__ import annotations
 
@@ -807,32 +807,20 @@ def run_e2e(texts: list, steps: int, warmup: int, world: int, dev):
 def run_reference(args, world, rank):
     """The reference's own CPU sorter on the same workload, on this host's cores: kolmo_sais_bwt_aux and
     kolmo_sais_unbwt_aux compiled from the reference's sources (oracle/Makefile) with every host thread, each step the
-    whole workload. Where that library is not available the CPU restatement runs on a bounded sample instead."""
+    whole workload. Where that library is not built the arm is unavailable: the restatement is not the reference."""
     if rank != 0:
         return None
     from kolmo_gb300.host import codec18_rlog
 
+    kind, fwd, inv, threads = cpu_sorter()
+    if kind != "reference":
+        return {"impl": "reference", "unavailable": "the reference's sorter is not built on this machine (its sources are "
+                                                    "not staged here)"}
     named, wname = single_blocks(args.workload if args.workload in ("markov1", "degenerate") else "prose64", 0,
                                  args.block_mib)
-    texts = [T for _, T in named]
-    kind, fwd, inv, threads = cpu_sorter()
-    if kind == "reference":
-        samples = texts
-        desc = (f"the whole workload ({sum(T.size for T in texts) / MIB:.0f} MiB) per step, forward+inverse, "
-                f"kolmo_sais_bwt_aux + kolmo_sais_unbwt_aux with threads={threads}")
-    else:
-        # size the per-step sample so that warm-up + steps stay within about two minutes
-        T = texts[0]
-        r = 1 << codec18_rlog(T.size)
-        probe = T[: 4 * MIB]
-        t0 = time.perf_counter()
-        rc, U, I = fwd(probe, r)
-        inv(U, r, I)
-        speed = probe.size / (time.perf_counter() - t0)  # bytes/s
-        per_step = 120.0 / max(args.steps + args.warmup, 1)
-        samples = [T[: int(min(T.size, max(4 * MIB, speed * per_step)))]]
-        desc = (f"first {samples[0].size / MIB:.1f} MiB of the first block per step, forward+inverse, r={r}; "
-                f"forward on one thread (SA-IS restatement), inverse on {threads} threads (per-sample decode)")
+    samples = [T for _, T in named]
+    desc = (f"the whole workload ({sum(T.size for T in samples) / MIB:.0f} MiB) per step, forward+inverse, "
+            f"kolmo_sais_bwt_aux + kolmo_sais_unbwt_aux with threads={threads}")
     rs = [1 << codec18_rlog(S.size) for S in samples]
     for _ in range(args.warmup):
         for S, r in zip(samples, rs):
@@ -851,9 +839,9 @@ def run_reference(args, world, rank):
             "steps": args.steps, "warmup": args.warmup, "ms_per_step": round(t / args.steps * 1e3, 2),
             "higher_is_better": True, "scaling": "weak", "vs_baseline": None, "dtype": "u8", "data": "synthetic",
             "impl": "reference",
-            "config": {"workload": wname, "bytes": int(sum(T.size for T in texts)),
+            "config": {"workload": wname, "bytes": int(total),
                        "blocks": [{"block": nm, "bytes": int(T.size), "r": 1 << codec18_rlog(int(T.size))}
-                                  for nm, T in named], "parallelism": "cpu", "same_config": kind == "reference"},
+                                  for nm, T in named], "parallelism": "cpu", "same_config": True},
             "cpu_baseline": {"value": round(v, 2), "unit": "MiB/s", "cores": threads, "kind": kind, "sample": desc},
             "e2e": {"value": round(v, 2), "unit": "MiB/s", "h2d_bytes_per_step": 0, "d2h_bytes_per_step": 0}}
 
