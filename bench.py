@@ -248,7 +248,7 @@ def single_blocks(workload: str, rank: int, mib: int):
 # case: profiles/traffic_group_thread_lsd_pass_prose16.md (tiny groups) and profiles/lsd_pass_prose16.md (the
 # round-0 radix pass, averaged over the 8 passes of coded keys). The 64 MiB launch's traffic is scaled by the suffixes it
 # processes.
-TRAFFIC_PER_SUFFIX = {"group_thread": 35.1, "lsd_pass": 15.0}
+TRAFFIC_PER_SUFFIX = {"group_thread": 32.8, "lsd_pass": 15.0}
 RANK_SORTERS = ("tile_sort_rank", "tile_warp_rank", "group_thread", "group_warp", "keygen")
 
 
@@ -901,7 +901,7 @@ def main():
     ap.add_argument("--small-group", type=int, default=-1)
     ap.add_argument("--warp-path", type=int, default=-1)
     ap.add_argument("--lsd-round0", type=int, default=-1)
-    ap.add_argument("--lsd-bytes", type=int, default=-1, help="prefix bytes of the LSD round 0 (8, 12 or 16)")
+    ap.add_argument("--lsd-bytes", type=int, default=-1, help="key of the LSD round 0: 12 or 16 bytes of text, or 8 of coded text")
     ap.add_argument("--chain-from", type=int, default=-1, help="first rank round with repeat chains (0: none)")
     ap.add_argument("--profile-out", default="", help="write the per-launch profile of the profiled step here")
     ap.add_argument("--plain", action="store_true",

@@ -769,7 +769,7 @@ int32_t kgbwt_engine_stats(kgbwt_engine *e, int32_t *rounds, int32_t *passes, in
     if (!e) return -1;
     if (e->last_kind == 2) {
         if (rounds) *rounds = 0;
-        if (passes) *passes = e->inv.stats.jumps;
+        if (passes) *passes = 1;  // one launch ranks the chains
         if (launches) *launches = e->inv.stats.launches;
         return 0;
     }

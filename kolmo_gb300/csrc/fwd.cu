@@ -2506,9 +2506,9 @@ int FwdEngine::run_plain(cudaStream_t s) {
     return 0;
 }
 
-// Graph: init -> round 0 -> while (active) { rank round } -> samples, where a round is
-//   fixup, keygen, msd_begin -> while (pass input non-empty) { hist, scan, scatter, msd_next } -> tiles, round_end.
-// Round 0 (prefix keys) is laid out once before the loop, the rank round is the loop body; the loops close with
+// Graph: init -> round 0 -> while (active) { rank round } -> samples. The bucket passes of a round are a loop of their own,
+// while (pass input non-empty) { hist, scan, scatter, msd_next }, beside the kernels of the lists that do not wait for
+// them (add_tile_round). Round 0 is laid out once before the loop, the rank round is the loop body; the loops close with
 // conditional while-nodes whose handles the 1-thread control kernels set.
 typedef std::vector<cudaGraphNode_t> Deps;
 

@@ -39,9 +39,17 @@ constexpr int ITPB = 256;
 constexpr u32 ITILE = 4096;
 constexpr u32 MARK = 64;
 // Small batches (the drop-in call on a block of a few MiB) mark more rows: they have too few chains to fill the GPU
-// otherwise, and their walk is as long as the longest chain, about MARK ln(chains) rows. Whole inverse, one row in 64
-// / 16 / 8 / 4: 20 KB - / 79 / 69 / 63 us, 1 MiB - / 115 / 103 / 115 us; at 30 MB one in 32 takes 0.10 ms off the walk and
-// adds as much to the ranking and the copies.
+// otherwise, and their walk is as long as the longest chain, about MARK ln(chains) rows. Whole inverse of one block, one
+// row in 4 / 8 / 16 / 32 / 64, us (the mean of log lines and Markov bytes):
+//    20 KB    61 / 67 / 79 / 94 / 172       768 KiB  98 / 92 / 111 / 136 / 197     3 MiB  213 / 162 / 162 / 188 / 271
+//   128 KiB   62 / 67 / 80 / 103 / 155      1 MiB   111 / 98 / 97 / 123 / 172      4 MiB  294 / 198 / 168 / 181 / 220
+//   192 KiB   68 / 76 / 94 / 120 / 180    1.5 MiB   137 / 117 / 128 / 148 / 225    5 MiB    - / - / 207 / 223 / 303
+//   256 KiB   66 / 70 / 85 / 111 / 171      2 MiB   178 / 130 / 128 / 144 / 196    8 MiB    - / - / 260 / 239 / 281
+//   512 KiB   82 / 76 / 86 / 119 / 168                                            16 MiB    - / - / 475 / 419 / 444
+// Both sides of each line: one in 4 stays ahead to about 300 KiB (6-12% between 128 KiB, where the line lies, and there),
+// 8 and 16 meet between 1 and 3 MiB, and past 4 MiB one in 16 or 32 would be ahead of 64 (46% at 5 MiB, 18% at 8, 6% at 16)
+// at two to four times the chain records. At 30 MB one in 32 takes 0.10 ms off the walk and adds as much to the ranking and
+// the copies.
 static u32 mark_of(u64 total) { return total <= 128u << 10 ? 4 : total <= 1536u << 10 ? 8 : total <= 4u << 20 ? 16 : MARK; }
 constexpr u32 CAPC = 256;
 constexpr u32 ENDC = 0xFFFFFFFFu;
@@ -345,7 +353,7 @@ __device__ __forceinline__ u32 walk_block(const InvArgs &a, u32 q) {
 // Chains that reach CAPC bytes continue under a new id taken from the block's counter. ONE: the batch is one block,
 // whose byte tables fit shared memory (a batch of several reads them through L1).
 //
-// Bound by dependent random psi loads: 77 G rows/s over the small blocks of a batch, 49 G on a 64 MiB block, whose
+// Bound by dependent random psi loads: 77 G rows/s over the small blocks of a batch, 50-55 G on a 64 MiB block, whose
 // 256 MiB table is twice L2 (independent 4-byte loads reach 79 G/s there, 280 where the table fits). One chain per
 // thread; CTA c takes runs c, c + G, c + 2G, ... of ITPB chains of the sequence, its threads the next of them as they
 // finish, so that the GPU works on one stretch of the sequence at a time. Chains are closed, stored and replaced only
@@ -739,7 +747,6 @@ int InvEngine::run(cudaStream_t s, bool use_graph) {
         KGB_CHECK(cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev));
         walk_grid = WALK_CTAS * sm_count;
     }
-    stats.jumps = 1;
     KGB_CHECK(cudaMemcpyAsync(d_blk, h_blk.data(), h_blk.size() * sizeof(InvBlock), cudaMemcpyHostToDevice, s));
     KGB_CHECK(cudaEventRecord(up_done, s));
     up_pending = true;

@@ -25,7 +25,6 @@ struct InvBlock {
 
 struct InvStats {
     long long launches;
-    int jumps;
 };
 
 class InvEngine {
@@ -53,7 +52,6 @@ class InvEngine {
     int grow(u64 ncap, u32 bcap, u64 tcap, u64 ccap, u64 pcap);
     template <typename Add>
     void layout(u64 ncap, u32 bcap, u64 tcap, u64 ccap, u64 pcap, Add add);
-    int build_graph(cudaStream_t s);
     int enqueue(cudaStream_t s, long long *launches);
     u32 nmax() const;
     int uploads_done();
