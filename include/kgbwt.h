@@ -221,7 +221,8 @@ uint64_t kgbwt_estimate_bytes(int32_t kind, const int32_t *n, const int32_t *r, 
  * worker; the first caller to find it idle runs the oldest pending call together with every later pending call of
  * the same direction, in arrival order, while their input stays within KGBWT_BATCH_MIB (environment, default 256)
  * MiB, and the other callers wait. A job's own failure (bad arguments, a string that is no BWT) stays with that job;
- * if the combined batch fails as a whole (device memory, a layout too large), each of its calls is run again alone.
+ * if the combined batch fails as a whole (device memory, a layout too large), each of its calls is run again alone (but
+ * not an in-place call once results have been written: it returns -2, as its input may be overwritten).
  * With KGBWT_STATS=<path> in the environment every batch appends one line to that file.
  * kgbwt_dropin_stats writes up to cap of: forward calls, forward batches, largest forward batch (calls), inverse
  * calls, inverse batches, largest inverse batch, combined batches retried call by call; returns 7. */

@@ -171,6 +171,7 @@ static void settle(cudaStream_t s) {
 }
 
 int run_fwd_jobs(Worker &C, kgbwt_fwd_job *jobs, int32_t count, uint32_t flags) {
+    C.delivering = false;
     std::vector<int> dev;
     std::vector<u32> n, r;
     for (int i = 0; i < count; i++) {
@@ -247,6 +248,7 @@ int run_fwd_jobs(Worker &C, kgbwt_fwd_job *jobs, int32_t count, uint32_t flags) 
         }
     }
     const u8 *SL = C.stage_L.p;
+    C.delivering = true;
     for (size_t k = 0; k < dev.size(); k++) {
         kgbwt_fwd_job &j = jobs[dev[k]];
         const u32 p0 = I[E.iouts()[k]];
@@ -274,6 +276,7 @@ int run_fwd_jobs(Worker &C, kgbwt_fwd_job *jobs, int32_t count, uint32_t flags) 
 }
 
 int run_inv_jobs(Worker &C, kgbwt_inv_job *jobs, int32_t count, uint32_t flags) {
+    C.delivering = false;
     std::vector<int> dev;
     std::vector<u32> n, p0;
     for (int i = 0; i < count; i++) {
@@ -336,6 +339,7 @@ int run_inv_jobs(Worker &C, kgbwt_inv_job *jobs, int32_t count, uint32_t flags) 
     if ((rc = E.fetch_status(s, st))) return fail(rc);
     int first = 0;
     const u8 *SL = C.stage_L.p;
+    C.delivering = true;
     for (size_t k = 0; k < dev.size(); k++) {
         kgbwt_inv_job &j = jobs[dev[k]];
         const u8 *src = SL;
@@ -488,6 +492,16 @@ static void log_batch(int kind, size_t calls, size_t jobs, u64 bytes, int rc, co
     }
 }
 
+// Whether a call's input and output share bytes (in-place calls are allowed).
+template <typename Job>
+static bool in_place(const Job *jobs, int32_t count) {
+    for (int32_t i = 0; i < count; i++) {
+        const uintptr_t t = (uintptr_t)jobs[i].T, u = (uintptr_t)jobs[i].U, n = jobs[i].n > 0 ? (uintptr_t)jobs[i].n : 0;
+        if (t < u + n && u < t + n) return true;
+    }
+    return false;
+}
+
 // Runs the calls `take` as one batch on the default worker (the caller is the leader and owns the worker).
 static void run_coalesced(Context &C, std::vector<Pending *> &take) {
     const int kind = take[0]->kind;
@@ -513,7 +527,8 @@ static void run_coalesced(Context &C, std::vector<Pending *> &take) {
                   : run_fwd_jobs(C.w, fj.data(), (int32_t)fj.size(), flags);
         // Per-job outcomes (bad arguments, a string that is no BWT) are in the jobs' rc and stay with their jobs. A
         // failure of the combined batch as a whole (device memory, a batch too large to lay out) fails every job:
-        // then each call runs again alone, so that a call's result never depends on what it was batched with.
+        // then each call runs again alone, so that a call's result never depends on what it was batched with. Only where
+        // the batch failed while it delivered results, an in-place call keeps the failure: its input may be overwritten.
         bool whole = rc == -2;
         if (rc && !whole) {
             whole = true;
@@ -523,10 +538,21 @@ static void run_coalesced(Context &C, std::vector<Pending *> &take) {
             std::lock_guard<std::mutex> lock(C.mu);
             C.retried++;
         }
+        const bool delivering = C.w.delivering;  // (of the combined batch)
         size_t k = 0;
         for (Pending *p : take) {
             bool failed = false;
-            if (whole) {
+            if (whole && delivering &&
+                (kind ? in_place((kgbwt_inv_job *)p->jobs, p->count) : in_place((kgbwt_fwd_job *)p->jobs, p->count))) {
+                for (int32_t i = 0; i < p->count; i++, k++) {
+                    const int32_t jr = kind ? ij[k].rc : fj[k].rc;
+                    if (kind) ((kgbwt_inv_job *)p->jobs)[i].rc = jr;
+                    else ((kgbwt_fwd_job *)p->jobs)[i].rc = jr;
+                }
+                p->rc = rc;
+                failed = true;
+            } else if (whole) {
+                k += (size_t)p->count;
                 p->rc = kind ? run_inv_jobs(C.w, (kgbwt_inv_job *)p->jobs, p->count, flags)
                              : run_fwd_jobs(C.w, (kgbwt_fwd_job *)p->jobs, p->count, flags);
                 failed = p->rc != 0;

@@ -33,6 +33,7 @@ struct Worker {
     kgbwt_engine eng;
     cudaStream_t stream = nullptr;
     Pinned stage_L, stage_I;  // results for pageable destinations; sampled indexes
+    bool delivering = false;  // the last batch got as far as writing results into its callers' buffers
     int init();                   // creates the stream on first use
     u64 device_bytes() const { return eng.fwd.workspace_bytes() + eng.inv.workspace_bytes(); }
     void release();               // frees both workspaces and the staging (the stream stays)

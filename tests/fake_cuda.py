@@ -1,6 +1,6 @@
 """Test infrastructure: a stand-in for the CUDA runtime, preloaded into a child process without a GPU. Asynchronous copies
 stay queued until something waits for the stream, kernels are not launched, read-backs of the control block say that the
-sort is done, and copies from or to chosen buffers fail."""
+sort is done, copies from or to chosen buffers fail, and waits can be held."""
 import os
 import subprocess
 import sys
@@ -20,6 +20,8 @@ FAKE = r"""
 #include <cstdint>
 #include <cstdlib>
 #include <cstring>
+#include <atomic>
+#include <unistd.h>
 #include <vector>
 struct dim3 { unsigned x, y, z; };
 namespace {
@@ -27,13 +29,14 @@ struct Op { void *dst; const void *src; size_t n; int fill; };
 std::vector<Op> ops;                   // queued, not yet done
 const char *bad = nullptr;             // copies from or to this buffer fail
 const uint32_t *samples = nullptr;     // what the read-back of the sampled indexes gives
-size_t nsamples = 0, ctl_size = 0, ctl_done = 0;
+size_t nsamples = 0, npair = 0, ctl_size = 0, ctl_done = 0;
 int last = 0, launches = 0;
+std::atomic<int> hold{0}, waiting{0};  // held: waits for a stream last until released (10 s at most)
 void drain() {
     for (const Op &o : ops) if (o.src) memcpy(o.dst, o.src, o.n); else memset(o.dst, o.fill, o.n);
     for (const Op &o : ops) {
         if (o.src && o.n == ctl_size) *(uint32_t *)((char *)o.dst + ctl_done) = 1;
-        if (samples && o.src && o.n == nsamples * 4) memcpy(o.dst, samples, o.n);
+        if (samples && o.src && (o.n == nsamples * 4 || o.n == npair * 4)) memcpy(o.dst, samples, o.n);
     }
     ops.clear();
 }
@@ -41,10 +44,13 @@ void drain() {
 extern "C" {
 void fake_setup(size_t size, size_t done) { ctl_size = size; ctl_done = done; }
 void fake_samples(const uint32_t *v, size_t n) { samples = v; nsamples = n; }
+void fake_pair(const uint32_t *v, size_t n) { samples = v; npair = n; }  // read-backs of this size too
 void fake_bad(const void *p) { bad = (const char *)p; }
 int fake_pending() { return (int)ops.size(); }
 void fake_drain() { drain(); }
 int fake_launches() { return launches; }
+void fake_hold(int on) { hold = on; }
+int fake_waiting() { return waiting; }
 
 int cudaMemcpyAsync(void *d, const void *s, size_t n, int, void *) {
     if (bad && (d == bad || s == bad)) return last = 1;
@@ -54,7 +60,13 @@ int cudaMemcpyAsync(void *d, const void *s, size_t n, int, void *) {
 int cudaMemsetAsync(void *d, int v, size_t n, void *) { ops.push_back({d, nullptr, n, v}); return 0; }
 int cudaMemcpy(void *d, const void *s, size_t n, int) { drain(); memcpy(d, s, n); return 0; }
 int cudaMemset(void *d, int v, size_t n) { drain(); memset(d, v, n); return 0; }
-int cudaStreamSynchronize(void *) { drain(); return 0; }
+int cudaStreamSynchronize(void *) {
+    waiting++;
+    for (int i = 0; hold && i < 10000; i++) usleep(1000);
+    waiting--;
+    drain();
+    return 0;
+}
 int cudaEventSynchronize(void *) { drain(); return 0; }
 int cudaMalloc(void **p, size_t n) { return (*p = calloc(n, 1)) ? 0 : 2; }
 int cudaFree(void *p) { free(p); return 0; }
